@@ -124,14 +124,29 @@ struct RayTiles {
     int tilesX;
     int count;
 };
-__global__ void raymarch(float4* out, ScalarFieldsIn s, Velocity vel, const float4* lightF, const float* shadowF, FrameParams p, RayTiles tiles);
+// Sin hashes of the raymarch's four fbm3 fields (kRenderOctaves octaves each),
+// built once per frame at every lattice point that the frame's samples can
+// reach: entry (x, y, z) of a table holds the hashes of the corners (0, 0),
+// (1, 0), (0, 1) and (1, 1) of the lattice cell's face at z.  sx = 0: the
+// octave has no table and is hashed in place.
+constexpr int kRenderOctaves = 3;
+constexpr int kRenderTables = 4 * kRenderOctaves;
+struct RenderNoise {
+    const float4* values;
+    int total;                                                                  // entries of all tables
+    int ox[kRenderTables], oy[kRenderTables], oz[kRenderTables];                // lattice point of entry (0, 0, 0)
+    int sx[kRenderTables], sy[kRenderTables], sz[kRenderTables], offset[kRenderTables];
+};
+__global__ void renderNoiseBuild(float4* values, RenderNoise T);
+__global__ void raymarch(float4* out, ScalarFieldsIn s, Velocity vel, const float4* lightF, const float* shadowF, FrameParams p, RayTiles tiles,
+                         RenderNoise noise);
 // The same for one scene id (0, 1, 2) fixed at compile time, without a debug view.
 __global__ void raymarchScene0(float4* out, ScalarFieldsIn s, Velocity vel, const float4* lightF, const float* shadowF, FrameParams p,
-                               RayTiles tiles);
+                               RayTiles tiles, RenderNoise noise);
 __global__ void raymarchScene1(float4* out, ScalarFieldsIn s, Velocity vel, const float4* lightF, const float* shadowF, FrameParams p,
-                               RayTiles tiles);
+                               RayTiles tiles, RenderNoise noise);
 __global__ void raymarchScene2(float4* out, ScalarFieldsIn s, Velocity vel, const float4* lightF, const float* shadowF, FrameParams p,
-                               RayTiles tiles);
+                               RayTiles tiles, RenderNoise noise);
 __global__ void emberSetup(EmberSplat* embers, ScalarFieldsIn s, Velocity vel, FrameParams p);
 __global__ void emberGather(float4* hdr, const EmberSplat* embers, FrameParams p);
 __global__ void tonemapOverlay(uint32_t* frame, const float4* hdr, FrameParams p, int doTonemap, int doOverlay);

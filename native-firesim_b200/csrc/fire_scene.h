@@ -216,6 +216,10 @@ private:
     float* sourceLattice_ = nullptr;
     size_t sourceCapacity_ = 0;
     // Raymarch work list: tile order (centre first) and the tile counter.
+    // Hash tables of the raymarch's noise fields, allocated by the first frame that uses them.
+    bool renderNoise(const FrameParams& p, RenderNoise& n);
+    float4* renderNoise_ = nullptr;
+    bool renderNoiseRefused_ = false;  // their allocation failed: frames hash in place
     int* rayTileOrder_ = nullptr;
     int* rayTileCounter_ = nullptr;
     int rayTilesX_ = 0, rayTileCount_ = 0;
