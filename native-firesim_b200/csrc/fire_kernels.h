@@ -239,11 +239,32 @@ constexpr int kMgCoarsestSweeps = 32;
 constexpr int kMgHardCycleCap = 1000;  // fireCudaSetPressureMultigrid accepts at most this many cycles
 constexpr unsigned kMgMaxPolls = 1u << 26;
 constexpr unsigned kMgStatusFlag = 0x80000000u;  // host status word: a multigrid barrier wait ran out (low bits: phase)
+// The smoothing's tile of a grid level (x a multiple of 4), whose region (the
+// tile and a halo of kMgPassHalves cells) is held in shared memory, p and rhs.
+constexpr int kMgPassHalves = 4;  // half sweeps of one smoothing pass, at most
+struct MgTile {
+    int x, y, z;
+};
+constexpr int kMgTileShapes = 4;
+constexpr MgTile kMgTiles[kMgTileShapes] = {{32, 16, 16}, {16, 16, 8}, {16, 8, 8}, {8, 8, 4}};
+inline long long mgTiles(const MgTile& t, const MgLevel& L) {
+    return static_cast<long long>((L.nx + t.x - 1) / t.x) * ((L.ny + t.y - 1) / t.y) * ((L.nz + t.z - 1) / t.z);
+}
+inline int mgTileCells(const MgTile& t) { return (t.x + 2 * kMgPassHalves) * (t.y + 2 * kMgPassHalves) * (t.z + 2 * kMgPassHalves); }
+// Passes of a smoothing of `halves` half sweeps, and of the post-smoothing: the
+// passes of a cycle alternate between a level's two buffers, so their number is
+// even.
+__host__ __device__ inline int mgSmoothPasses(int halves) { return (halves + kMgPassHalves - 1) / kMgPassHalves; }
+__host__ __device__ inline int mgPostPasses(int pre, int post) {
+    const int passes = mgSmoothPasses(2 * post);
+    return passes + ((mgSmoothPasses(2 * pre) + passes) & 1);
+}
 // One scene of a solve.  Level l's p and rhs: level 0 is the increment and
 // the divergence array; levels >= 1 are the coarse corrections.
 struct MgScene {
     MgLevel lv[kMgMaxLevels];
     float* p[kMgMaxLevels];
+    float* q[kMgMaxLevels];    // the smoothing's other buffer of each grid level
     float* rhs[kMgMaxLevels];
     float* pressure;   // += the increment at the end of the solve
     SorGate* gate;     // zeroed before the launch
@@ -253,21 +274,22 @@ struct MgScene {
     int tailMode;      // MgTailMode
 };
 // The work lists of a solve, as prefix sums over the scenes (0 for a scene
-// whose tail starts at or above the level).  smoothUnits and fineUnits count
-// the units of grid level l (the smoothing's and the prolongation's): where
-// the row length is a multiple of 4, 128 consecutive cells in memory, four
-// per lane (mgQuadUnits); otherwise 128-cell (smoothing) or 32-cell
-// (prolongation) chunks of single rows.  coarseUnits counts the restriction's
+// whose tail starts at or above the level).  tileUnits counts the smoothing's
+// tiles of grid level l, fineUnits the prolongation's units: where the row
+// length is a multiple of 4, 128 consecutive cells in memory, four per lane
+// (mgQuadUnits); otherwise 32-cell chunks of single rows.  coarseUnits counts the restriction's
 // units of level l + 1: 64 consecutive coarse cells where the fine row length
 // is a multiple of 4, else 32-cell chunks of single rows.  chunks counts the
 // residual's chunks of level 0 (mgResidualChunks), allUnits the units of
-// level 0 as the smoothing takes them (for the first and last phases).
+// level 0 of the first and last phases: 128 consecutive cells where the row
+// length is a multiple of 4, else 128-cell chunks of single rows.
 struct MgPlan {
     int scenes;
     int gridLevels;  // max over the scenes of tail
     int maxCycles, pre, post, gated;
     float tolerance;
-    int smoothUnits[kMgMaxLevels][kMgMaxScenes + 1];
+    int tile[kMgMaxLevels];  // index of the level's tile shape in kMgTiles
+    int tileUnits[kMgMaxLevels][kMgMaxScenes + 1];
     int fineUnits[kMgMaxLevels][kMgMaxScenes + 1];
     int coarseUnits[kMgMaxLevels][kMgMaxScenes + 1];
     int chunks[kMgMaxScenes + 1];

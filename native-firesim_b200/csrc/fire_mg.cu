@@ -30,8 +30,10 @@
 // One launch (mgSolve) runs every cycle of every scene of the batch.  Its
 // CTAs are all co-resident (cooperative launch); the phases of a cycle are
 // separated by a grid barrier (a monotonic arrival count with release and
-// acquire semantics) whose waits are bounded in time.  Within a phase, warps
-// take the units of all scenes at that level from one work list.  A level's
+// acquire semantics) whose waits are bounded in time.  A smoothing runs up to
+// four half sweeps per phase on tiles in shared memory, a CTA per tile; in the
+// other phases warps take the units of all scenes at that level from one work
+// list.  A level's
 // first colour-0 half sweep from p = 0 is written with its rhs (by the
 // restriction, or the first phase for level 0 in the first cycle), as its
 // arithmetic reduces to (rhs + 0) / diag there.
@@ -509,10 +511,188 @@ __device__ __forceinline__ float quadSum(const MgLevel& L, const Quad& q, int e,
     return combine(at4(q.rh, e), pL, pR, pD, pU, pB, pF, L);
 }
 
-// Asks L2 to fetch the line holding a (no register or shared memory holds
-// the data; the load that follows finds it there).
-__device__ __forceinline__ void prefetchLineL2(const float* a) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(a)));
+// ---- smoothing: up to four half sweeps of one tile in shared memory -------
+// A half sweep over global memory reads p (with its neighbours) and the rhs and
+// writes p through L2 for two flops a byte, and costs a grid barrier: 8.7 us at
+// 128^3 (of it 2.3 us of barrier), 45 us at 256^3, 3.8 us (2.1) at 32^3.  Four of
+// them as one phase of tiles take 24.5, 169 and 5.7 us; a tile of 32x16x16 cells
+// 2.9 us to load, 5.7 us for its four half sweeps (shared memory: 5.8 updates per
+// wavefront) and 0.7 us to store.  A V-cycle went 208 -> 169 us at 128^3, 711 ->
+// 671 us at 256^3 and 119 -> 93 us at 64^3.
+//
+// A CTA loads a tile of p and the rhs with a halo of four cells, runs `count`
+// half sweeps on it (each valid one cell less far into the halo) and writes the
+// tile's own cells to the level's other buffer, so that neighbouring tiles
+// still find the old halo.  Per cell the arithmetic and its order are
+// weightedSum's.
+//
+// Shared memory holds p and the rhs split by colour: colour c, row (y, z), slot
+// k holds x = 2 k + ((c + y + z) & 1), so every neighbour of a cell is of the
+// other colour in the same slot or the one beside it, and lanes over slots do
+// not conflict.  A thread walks the columns of two slots (y; k, k + 1) along z
+// with the other colour's values below, here and above in registers; GROUPS
+// threads share them.  The shape is a compile-time constant, so that every
+// operand is a fixed offset from the column's address.  Cells of the halo past
+// a half sweep's reach in x, and slots outside the grid, are updated too: they
+// get values that no valid cell reads.
+template <int TX, int TY, int TZ>
+struct TileShape {
+    static constexpr int H = kMgPassHalves;
+    static constexpr int QUADS = (TX + 2 * H) / 4, K = 2 * QUADS;  // quads and slots of a region row
+    static constexpr int RY = TY + 2 * H, RZ = TZ + 2 * H;
+    static constexpr int PLANE = RY * K, COLOUR = RZ * PLANE;
+    static constexpr int COLS = RY * QUADS;
+    static constexpr int GROUPS = kMgThreads / COLS;
+    static constexpr int LOADS = QUADS * RY * RZ;
+    static_assert(GROUPS >= 1 && 2 * COLOUR == (TX + 2 * H) * RY * RZ, "tile shape");
+};
+
+__device__ __forceinline__ float2 at2(const float* a) { return *reinterpret_cast<const float2*>(a); }
+
+// Half sweep `colour` of a loaded tile on the rows and planes at most `margin`
+// outside it.
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ void tileHalfSweep(const MgLevel& L, float* smem, int x0, int y0, int z0, int colour, int margin) {
+    using S = TileShape<TX, TY, TZ>;
+    const int group = threadIdx.x / S::COLS, col = threadIdx.x - group * S::COLS;
+    if (group >= S::GROUPS) return;
+    const int ly = col / S::QUADS, q = col - ly * S::QUADS;
+    const int y = y0 - S::H + ly, x = x0 - S::H + 4 * q;  // the first slot's x is x + shift, the second's x + 2 + shift
+    const int zLo = max(z0 - margin, 0), zHi = min(z0 + TZ + margin, L.nz);
+    const int per = (zHi - zLo + S::GROUPS - 1) / S::GROUPS;
+    const int zA = zLo + group * per, zB = min(zA + per, zHi);
+    if (y < max(y0 - margin, 0) || y >= min(y0 + TY + margin, L.ny) || zA >= zB) return;
+    // The columns' cells of the colour and of the other one, at plane zA.
+    const int first = (zA - z0 + S::H) * S::PLANE + ly * S::K + 2 * q;
+    float* own = smem + colour * S::COLOUR + first;
+    const float* other = smem + (1 - colour) * S::COLOUR + first;
+    // Walls in y: the cell itself, and its negative above the top row.
+    const bool top = y == L.ny - 1;
+    const float* down = y == 0 ? own : other - S::K;
+    const float* up = top ? own : other + S::K;
+    // The x neighbours of slot i are the other colour's slots i - 1 and i (shift
+    // 0) or i and i + 1: of the two cells one has the two slots here, the other
+    // one of them and the slot before or after, at a wall the cell itself.
+    bool after = ((colour + y + zA) & 1) != 0;  // shift 1 at this plane
+    const float* sideBefore = x == 0 ? own : other - 1;
+    const float* sideAfter = x + 3 == L.nx - 1 ? own + 1 : other + 2;
+    const float *side = after ? sideAfter : sideBefore, *sideNext = after ? sideBefore : sideAfter;
+    // nx odd: a cell of shift 0 at x = nx - 1, in slot 0 or 1; nx - 1 = x + 1 in slot 0 with shift 1.
+    const bool end0 = x == L.nx - 1, end1 = x + 2 == L.nx - 1, end2 = x + 1 == L.nx - 1;
+    const bool odd = end0 || end1 || end2;
+    float2 below = zA == 0 ? at2(own) : at2(other - S::PLANE);
+    float2 here = at2(other);
+    auto update = [&](int o, const float* side, bool after, float2 above) {
+        const float2 d = at2(down + o), u = at2(up + o), b = at2(own + o + 2 * S::COLOUR);
+        const float pair = here.x + here.y;
+        const float edge = side[o] + (after ? here.y : here.x);
+        float lat0 = after ? pair : edge, lat1 = after ? edge : pair;
+        if (odd) {
+            const float2 self = at2(own + o);
+            if (!after && end0) lat0 = side[o] + self.x;
+            if (!after && end1) lat1 = here.x + self.y;
+            if (after && end2) lat0 = here.x + self.x;
+        }
+        float2 r;
+        r.x = (b.x + L.wx * lat0 + L.wy * (d.x + (top ? 0.0f - u.x : u.x)) + L.wz * (below.x + above.x)) * L.invDiag;
+        r.y = (b.y + L.wx * lat1 + L.wy * (d.y + (top ? 0.0f - u.y : u.y)) + L.wz * (below.y + above.y)) * L.invDiag;
+        *reinterpret_cast<float2*>(own + o) = r;
+        below = here;
+        here = above;
+    };
+    const int count = min(zB, L.nz - 1) - zA;  // planes with a plane above them
+    int n = 0;
+    for (; n + 1 < count; n += 2) {
+        update(0, side, after, at2(other + S::PLANE));
+        update(S::PLANE, sideNext, !after, at2(other + 2 * S::PLANE));
+        own += 2 * S::PLANE;
+        other += 2 * S::PLANE;
+        down += 2 * S::PLANE;
+        up += 2 * S::PLANE;
+        side += 2 * S::PLANE;
+        sideNext += 2 * S::PLANE;
+    }
+    if (n < count) {
+        update(0, side, after, at2(other + S::PLANE));
+        if (zB == L.nz) update(S::PLANE, sideNext, !after, at2(own + S::PLANE));
+    } else if (zB == L.nz) {
+        update(0, side, after, at2(own));
+    }
+}
+
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void tileSmooth(const MgLevel& level, const float* __restrict__ src, const float* __restrict__ rhs,
+                                        float* __restrict__ dst, int tile, int first, int count) {
+    using S = TileShape<TX, TY, TZ>;
+    extern __shared__ float smem[];  // [p, rhs][colour][RZ][RY][K]
+    const MgLevel L = level;
+    const int tilesX = (L.nx + TX - 1) / TX, tilesY = (L.ny + TY - 1) / TY;
+    const int tz = tile / (tilesX * tilesY), ty = (tile - tz * tilesX * tilesY) / tilesX, tx = tile - (tz * tilesY + ty) * tilesX;
+    const int x0 = tx * TX, y0 = ty * TY, z0 = tz * TZ;
+    const bool whole = (L.nx & 3) == 0;
+    constexpr int BATCH = 3;  // quads in flight per thread
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < S::LOADS; i0 += BATCH * kMgThreads) {
+        float4 p[BATCH], r[BATCH];
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+            const int i = i0 + j * kMgThreads;
+            const int row = i / S::QUADS, q = i - row * S::QUADS;
+            const int lz = row / S::RY, ly = row - lz * S::RY;
+            const int x = x0 - S::H + 4 * q, y = y0 - S::H + ly, z = z0 - S::H + lz;
+            const bool in = i < S::LOADS && x >= 0 && x < L.nx && y >= 0 && y < L.ny && z >= 0 && z < L.nz;
+            const int g = (z * L.ny + y) * L.nx + x;
+            p[j] = r[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (in && whole) {
+                p[j] = ldcg4(src + g);
+                r[j] = ldcg4(rhs + g);
+            } else if (in) {
+                const float* a = src + g;
+                const float* b = rhs + g;
+                const int n = L.nx - x;
+                p[j] = make_float4(__ldcg(a), n > 1 ? __ldcg(a + 1) : 0.0f, n > 2 ? __ldcg(a + 2) : 0.0f, n > 3 ? __ldcg(a + 3) : 0.0f);
+                r[j] = make_float4(__ldcg(b), n > 1 ? __ldcg(b + 1) : 0.0f, n > 2 ? __ldcg(b + 2) : 0.0f, n > 3 ? __ldcg(b + 3) : 0.0f);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+            const int i = i0 + j * kMgThreads;
+            if (i >= S::LOADS) break;
+            const int row = i / S::QUADS, q = i - row * S::QUADS;
+            const int lz = row / S::RY, ly = row - lz * S::RY;
+            const int even = (y0 + ly + z0 + lz) & 1;  // the colour of the row's even cells (the halo is even)
+            float* e = smem + even * S::COLOUR + row * S::K + 2 * q;
+            float* o = smem + (1 - even) * S::COLOUR + row * S::K + 2 * q;
+            *reinterpret_cast<float2*>(e) = make_float2(p[j].x, p[j].z);
+            *reinterpret_cast<float2*>(o) = make_float2(p[j].y, p[j].w);
+            *reinterpret_cast<float2*>(e + 2 * S::COLOUR) = make_float2(r[j].x, r[j].z);
+            *reinterpret_cast<float2*>(o + 2 * S::COLOUR) = make_float2(r[j].y, r[j].w);
+        }
+    }
+    __syncthreads();
+    for (int s = 0; s < count; ++s) {
+        tileHalfSweep<TX, TY, TZ>(L, smem, x0, y0, z0, (first + s) & 1, count - 1 - s);
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < TX / 4 * TY * TZ; i += kMgThreads) {
+        const int row = i / (TX / 4), q = i - row * (TX / 4);
+        const int lz = row / TY, ly = row - lz * TY;
+        const int x = x0 + 4 * q, y = y0 + ly, z = z0 + lz;
+        if (x >= L.nx || y >= L.ny || z >= L.nz) continue;
+        const int g = (z * L.ny + y) * L.nx + x;
+        const int even = (y + z) & 1;
+        const int at = ((lz + S::H) * S::RY + ly + S::H) * S::K + 2 * q + S::H / 2;
+        const float2 e = at2(smem + even * S::COLOUR + at), o = at2(smem + (1 - even) * S::COLOUR + at);
+        if (whole) {
+            *reinterpret_cast<float4*>(dst + g) = make_float4(e.x, o.x, e.y, o.y);
+        } else {
+            dst[g] = e.x;
+            if (x + 1 < L.nx) dst[g + 1] = o.x;
+            if (x + 2 < L.nx) dst[g + 2] = e.y;
+            if (x + 3 < L.nx) dst[g + 3] = o.y;
+        }
+    }
+    __syncthreads();
 }
 
 // Coordinates of flat index i of a level.
@@ -559,67 +739,41 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     }
     __syncthreads();
     auto converged = [&](int s) { return sRunning[s] == 0; };
-    // One colour of red-black Gauss-Seidel on level l of every scene that has
-    // it as a grid level.  Where the row length is a multiple of 4, a unit is
-    // 128 consecutive cells in memory (several short rows, or part of a long
-    // one), four per lane: each lane updates the two of its four cells of the
-    // colour and stores all four (the other two unchanged: no thread writes
-    // them in this phase).  Otherwise a unit is a 128-cell chunk of one row,
-    // taken cell by cell.
-    auto smooth = [&](int l, int colour) {
-        const int* off = plan->smoothUnits[l];
+    // Half sweeps first .. first + count - 1 (count <= kMgPassHalves) of level l
+    // of every scene that has it as a grid level, one tile per CTA at a time.
+    // The results go to the level's other buffer (side: 0 if they come from p).
+    auto smooth = [&](int l, int first, int count, int side) {
+        const int* off = plan->tileUnits[l];
         const int total = __ldg(off + n);
-        for (int unit = gwarp; unit < total; unit += nwarps) {
+        const int shape = __ldg(&plan->tile[l]);
+        for (int unit = blockIdx.x; unit < total; unit += gridDim.x) {
             const int s = sceneOf(off, n, unit);
             if (converged(s)) continue;
             const MgScene& S = scenes[s];
-            const MgLevel L = S.lv[l];
-            const int u = unit - __ldg(off + s);
-            float* p = S.p[l];
-            const float* rhs = S.rhs[l];
-            if ((L.nx & 3) == 0) {
-                const int i = u * 128 + 4 * lane;
-                const bool live = i < L.nx * L.ny * L.nz;
-                // Ask L2 for this lane's cells of the warp's next unit (when it
-                // is in the same scene), so that its loads find them there.
-                const int ahead = i + nwarps * 128;
-                if (ahead < L.nx * L.ny * L.nz) {
-                    prefetchLineL2(rhs + ahead);
-                    prefetchLineL2(p + ahead);
-                }
-                int x0, y, z;
-                flatCoords(L, live ? i : 0, x0, y, z);
-                Quad q;
-                quadLoad(q, p, rhs, l == 0, L, i, x0, y, z, lane, live);
-                if (!live) continue;
-                const int e0 = (colour + x0 + y + z) & 1;  // the colour's cells are e0 and e0 + 2
-                const float a = quadSum(L, q, e0, x0 + e0, y, z) * L.invDiag;
-                const float b = quadSum(L, q, e0 + 2, x0 + e0 + 2, y, z) * L.invDiag;
-                float4 o = q.c;
-                if (e0 == 0) {
-                    o.x = a;
-                    o.z = b;
-                } else {
-                    o.y = a;
-                    o.w = b;
-                }
-                *reinterpret_cast<float4*>(p + i) = o;
+            const int tile = unit - __ldg(off + s);
+            const float* src = side ? S.q[l] : S.p[l];
+            float* dst = side ? S.p[l] : S.q[l];
+            if (shape == 0) {
+                tileSmooth<32, 16, 16>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+            } else if (shape == 1) {
+                tileSmooth<16, 16, 8>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+            } else if (shape == 2) {
+                tileSmooth<16, 8, 8>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
             } else {
-                const int cpr = mgQuadChunks(L.nx);
-                const int row = u / cpr, chunk = u - row * cpr;
-                const int y = row % L.ny, z = row / L.ny;
-                const int base = row * L.nx;
-                auto load = [&](int j) { return __ldcg(p + j); };
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int x = chunk * 128 + 4 * lane + e;
-                    if (x >= L.nx || ((colour + x + y + z) & 1) != 0) continue;
-                    const int i = base + x;
-                    const float rh = l == 0 ? __ldg(rhs + i) : __ldcg(rhs + i);
-                    p[i] = weightedSum(load, rh, L, i, x, y, z, load(i)) * L.invDiag;
-                }
+                tileSmooth<8, 8, 4>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
             }
         }
+    };
+    // A smoothing of `halves` half sweeps from half sweep `first` on, in
+    // `passes` passes of about equal length.
+    auto smoothLevel = [&](int l, int first, int halves, int passes, int& side) {
+        for (int k = 0; k < passes; ++k) {
+            const int from = halves * k / passes, to = halves * (k + 1) / passes;
+            smooth(l, first + from, to - from, side);
+            side ^= 1;
+            if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return false;
+        }
+        return true;
     };
     // Coarse rhs = the mean residual of the covered fine cells, and coarse p
     // = 0, or, when `red` (the coarse level is a grid level whose
@@ -630,7 +784,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     // consecutive coarse cells in memory, two per lane, whose fine quad is
     // loaded row by row (quadLoad) for each of the fine rows covered;
     // otherwise a unit is a 32-cell chunk of a coarse row, a cell per lane.
-    auto restrictTo = [&](int l, bool redFirst) {
+    auto restrictTo = [&](int l, bool redFirst, int side) {
         const int* off = plan->coarseUnits[l];
         const int total = __ldg(off + n);
         for (int unit = gwarp; unit < total; unit += nwarps) {
@@ -640,7 +794,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             const MgLevel F = S.lv[l], C = S.lv[l + 1];
             const bool red = redFirst && l + 1 < S.tail;
             const int u = unit - __ldg(off + s);
-            const float* pf = S.p[l];
+            const float* pf = side ? S.q[l] : S.p[l];
             const float* rf = S.rhs[l];
             if ((F.nx & 3) == 0) {
                 const int j = u * 64 + 2 * lane;
@@ -698,7 +852,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     // the lane loads the coarse values at x0/2 and x0/2 + 1 and takes those
     // at x0/2 - 1 and x0/2 + 2 from the lanes beside it (clamped at the row's
     // ends).  Otherwise a unit is a 32-cell chunk of a row, a cell per lane.
-    auto prolongFrom = [&](int l) {
+    auto prolongFrom = [&](int l, int side) {
         const int* off = plan->fineUnits[l];
         const int total = __ldg(off + n);
         for (int unit = gwarp; unit < total; unit += nwarps) {
@@ -707,7 +861,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             const MgScene& S = scenes[s];
             const MgLevel F = S.lv[l], C = S.lv[l + 1];
             const int u = unit - __ldg(off + s);
-            float* pf = S.p[l];
+            float* pf = side ? S.q[l] : S.p[l];
             const float* pc = S.p[l + 1];
             if ((F.nx & 3) == 0) {
                 const int i = u * 128 + 4 * lane;
@@ -781,6 +935,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     // restrictTo: (rhs + 0) / diag on colour-0 cells, 0 elsewhere (scenes
     // whose level 0 is in the tail start from 0).  Units as the smoothing's.
     const bool redFirst = pre > 0;
+    const int prePasses = mgSmoothPasses(2 * pre), postPasses = mgPostPasses(pre, post);
     {
         const int total = __ldg(plan->allUnits + n);
         for (int unit = gwarp; unit < total; unit += nwarps) {
@@ -828,11 +983,10 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
         for (int l = 0; l < gridLevels; ++l) {
             // The colour-0 half sweep of a coarse level, and of level 0 in the
             // first cycle, was done with the restriction (the initialisation).
-            for (int k = redFirst && (l > 0 || cycle == 0) ? 1 : 0; k < 2 * pre; ++k) {
-                smooth(l, k & 1);
-                if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
-            }
-            restrictTo(l, redFirst);
+            const int done = redFirst && (l > 0 || cycle == 0) ? 1 : 0;
+            int side = 0;
+            if (!smoothLevel(l, done, 2 * pre - done, prePasses, side)) return;
+            restrictTo(l, redFirst, side);
             if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
         }
         for (int s = blockIdx.x; s < n; s += gridDim.x) {
@@ -850,12 +1004,10 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
         }
         if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
         for (int l = gridLevels - 1; l >= 0; --l) {
-            prolongFrom(l);
+            int side = prePasses & 1;
+            prolongFrom(l, side);
             if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
-            for (int k = 0; k < 2 * post; ++k) {
-                smooth(l, k & 1);
-                if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
-            }
+            if (!smoothLevel(l, 0, 2 * post, postPasses, side)) return;
         }
         if (gated) {
             // Level-0 residual, one warp per chunk (mgResidualChunk: a fixed

@@ -821,6 +821,30 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
         const MgLevel& L0 = scenes[s].lv[0];
         plan.allUnits[s + 1] = plan.allUnits[s] + ((L0.nx & 3) == 0 ? mgQuadUnits(L0.nx, L0.ny, L0.nz) : rows0 * mgQuadChunks(L0.nx));
     }
+    // The smoothing's tile of each grid level: of the shapes the one whose waves
+    // of tiles (a tile per CTA) take the least time, as a fixed latency of 1.5 us
+    // plus a time per cell of the region (measured: 9.3 us for 32x16x16's 23,040).
+    // Large tiles waste the least on halos; where they would leave SMs idle or
+    // end in a nearly empty wave, smaller ones finish sooner (32^3: 8x8x4 3.6 us).
+    for (int l = 0; l < plan.gridLevels; ++l) {
+        double best = 0.0;
+        for (int k = 0; k < kMgTileShapes; ++k) {
+            long long tiles = 0;
+            for (int s = 0; s < n; ++s) {
+                if (l < scenes[s].tail) tiles += mgTiles(kMgTiles[k], scenes[s].lv[l]);
+            }
+            const double cost = static_cast<double>((tiles + sms_ - 1) / sms_) * (1.5 + 3.4e-4 * mgTileCells(kMgTiles[k]));
+            if (best == 0.0 || cost < best) {
+                best = cost;
+                plan.tile[l] = k;
+            }
+        }
+        const MgTile& t = kMgTiles[plan.tile[l]];
+        for (int s = 0; s < n; ++s) {
+            plan.tileUnits[l][s + 1] = plan.tileUnits[l][s] + (l < scenes[s].tail ? static_cast<int>(mgTiles(t, scenes[s].lv[l])) : 0);
+        }
+        smem = std::max(smem, 2 * sizeof(float) * static_cast<size_t>(mgTileCells(t)));
+    }
     std::memcpy(hScenes, scenes.data(), n * sizeof(MgScene));
     int perSm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, mgSolve, kMgThreads, smem);
@@ -834,8 +858,6 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
             const bool grid = l < S.tail;
             const MgLevel& F = S.lv[l];
             const bool quad = (F.nx & 3) == 0;
-            const int units = quad ? mgQuadUnits(F.nx, F.ny, F.nz) : F.ny * F.nz * mgQuadChunks(F.nx);
-            plan.smoothUnits[l][s + 1] = plan.smoothUnits[l][s] + (grid ? units : 0);
             const int fine = quad ? mgQuadUnits(F.nx, F.ny, F.nz) : F.ny * F.nz * mgRowChunks(F.nx);
             plan.fineUnits[l][s + 1] = plan.fineUnits[l][s] + (grid ? fine : 0);
             if (grid) {
@@ -919,10 +941,16 @@ bool Scene::multigridScene(MgScene& out, std::string& err) {
     MgScene S{};
     S.levels = static_cast<int>(mgLevels_.size());
     S.tail = S.levels - 1;
+    size_t scratch = 0;
     for (int l = 0; l < S.levels; ++l) {
         S.lv[l] = mgLevels_[l];
         S.p[l] = mgP_[l];
         S.rhs[l] = l == 0 ? divergence_ : mgRhs_[l];
+        // The smoothing's other buffers, in the force scratch, which no stage of
+        // the projection uses: 16 B per cell, at most half of it needed (every
+        // level has at most half the cells of the one above).
+        S.q[l] = reinterpret_cast<float*>(contrib_) + scratch;
+        scratch += (static_cast<size_t>(mgLevels_[l].nx) * mgLevels_[l].ny * mgLevels_[l].nz + 3) & ~static_cast<size_t>(3);
         if (S.tail == S.levels - 1 && static_cast<long long>(mgLevels_[l].nx) * mgLevels_[l].ny * mgLevels_[l].nz <= kMgTailCells) {
             S.tail = l;
         }
