@@ -1051,8 +1051,9 @@ bool Scene::sourceLattice(const FrameParams& p, HashLattice2& l) const {
 // The tables of the raymarch's noise fields for this frame: per field and
 // octave every lattice cell that a sample position in [0, 1]^3 can reach, one
 // cell wider on each side (a cell outside is hashed in place, so the margin
-// affects speed only).  The sizes do not depend on the time, so one buffer
-// serves every frame; it is allocated by the first frame that uses it, and a
+// affects speed only).  The sizes do not depend on the time (1.46 M entries).
+// They lie in the force scratch, which no stage of a frame uses, where the grid
+// has that many cells; else in a buffer that the first frame allocates, and a
 // frame goes without where that fails or the stream is being captured.
 // The finest octave of the finest field has no table: its 7 M cells are 111 MB
 // more per scene, and hashing them costs what they save (render with and
@@ -1088,6 +1089,11 @@ bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
             n.offset[k] = total;
             total += n.sx[k] * n.sy[k] * n.sz[k];
         }
+    }
+    if (cells_ >= static_cast<size_t>(total)) {
+        n.values = contrib_;
+        n.total = total;
+        return true;
     }
     if (renderNoise_ == nullptr) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1197,7 +1203,7 @@ bool Scene::runStages(int first, int last, const FrameParams& p, std::string& er
                 auto kernel = k == 1 ? raymarchScene0 : (k == 2 ? raymarchScene1 : (k == 3 ? raymarchScene2 : raymarch));
                 RenderNoise noise{};
                 if (renderNoise(p, noise)) {
-                    renderNoiseBuild<<<1184, 256, 0, stream>>>(renderNoise_, noise); ++launches_;
+                    renderNoiseBuild<<<1184, 256, 0, stream>>>(const_cast<float4*>(noise.values), noise); ++launches_;
                 } else {
                     noise = RenderNoise{};
                 }
