@@ -252,12 +252,13 @@ FIRE_API bool fireCudaGetLaunchCount(unsigned long long* count);
  * at most 65535.
  *
  * Limit: at most 1,048,576 cells (nx*ny*nz); larger grids are rejected.  The
- * per-cell increments live in one fixed 16 MiB array that every GPU loading
- * the library holds until exit.  The first call on each device resolves that
- * array's device address, so make it before any stream capture.  All calls
- * share the array: calls that overlap on the GPU (other streams, other host
- * threads) race.  Each call overwrites the first nx*ny*nz entries before
- * reading them, so nothing has to be cleared between calls. */
+ * per-cell increments live in one fixed 16 MiB array, and the curl noise's hash
+ * lattices in one of 0.9 MiB, that every GPU loading the library holds until
+ * exit.  The first call on each device resolves their device addresses, so make
+ * it before any stream capture.  All calls share the arrays: calls that overlap
+ * on the GPU (other streams, other host threads) race.  Each call overwrites
+ * the entries that it reads before reading them, so nothing has to be cleared
+ * between calls. */
 FIRE_API bool fireCudaForceProjectNoAlloc(const FireSettings* settings, float time, int nx, int ny, int nz,
                                           const void* recordsA, const void* recordsB, const void* recordsC,
                                           const float* u, const float* v, const float* w, float* uOut, float* vOut,

@@ -6,8 +6,9 @@
 // of device memory through its own arena, a caller capturing its frame into a
 // CUDA graph (cudaMalloc is not capturable), or a plugin whose host forbids
 // third-party allocations after start-up.  fireCudaForceProjectNoAlloc runs
-// the same two kernels (forceContributions, forceProjectSetup) on buffers the
-// caller owns, and keeps the increments in the fixed array below instead.
+// the same kernels (hashLatticeBuild, forceContributions, forceProjectSetup) on
+// buffers the caller owns, and keeps the increments and the lattices in the
+// fixed arrays below instead.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -23,9 +24,18 @@ namespace {
 // cells: 16 MiB, held by every GPU that loads the library until the process exits.
 constexpr int kNoAllocMaxCells = 1 << 20;
 static __device__ __align__(256) float4 g_forceScratch[kNoAllocMaxCells];
+// The curl noise's hash lattices of one call (0.8 MiB): every call that uses them
+// builds them before reading them.
+static __device__ __align__(256) float g_curlLattice[2 * firesim::kCurlLatticeEntries];
 
-// Device address of g_forceScratch per device ordinal.  In host code the
-// symbol is only a host-side stand-in, so the address is resolved with
+// From this many cells on a call builds the lattices instead of hashing 40
+// corners per cell in place: a call on 120x88x96 cells 129 -> 56 us, 64^3 43 ->
+// 29 us, 40^3 25 -> 21 us; below, the launch costs more than the hashes (32^3
+// 17 us in place, 21 us with lattices).
+constexpr long long kLatticeMinCells = 48000;
+
+// Device addresses of the two arrays per device ordinal.  In host code a symbol
+// is only a host-side stand-in, so an address is resolved with
 // cudaGetSymbolAddress on each device, once, while that device is current.
 // Several host threads may resolve it at once; they store the same value, and
 // the atomics keep that free of data races.  A cudaDeviceReset (or a reset of
@@ -33,6 +43,7 @@ static __device__ __align__(256) float4 g_forceScratch[kNoAllocMaxCells];
 // after one: a process that resets a device must reload the library.
 constexpr int kMaxDevices = 64;
 std::atomic<float4*> g_scratchAddress[kMaxDevices] = {};
+std::atomic<float*> g_latticeAddress[kMaxDevices] = {};
 
 }  // namespace
 
@@ -97,6 +108,15 @@ extern "C" bool fireCudaForceProjectNoAlloc(const FireSettings* settings, float 
         g_scratchAddress[device].store(scratch, std::memory_order_release);
     }
 
+    float* lattice = g_latticeAddress[device].load(std::memory_order_acquire);
+    if (lattice == nullptr) {
+        void* addr = nullptr;
+        e = cudaGetSymbolAddress(&addr, g_curlLattice);
+        if (e != cudaSuccess) return fail(std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
+        lattice = static_cast<float*>(addr);
+        g_latticeAddress[device].store(lattice, std::memory_order_release);
+    }
+
     // The settings clamps of a step; Scene allocates nothing until init().
     firesim::Scene dims;
     dims.nx = nx;
@@ -113,9 +133,21 @@ extern "C" bool fireCudaForceProjectNoAlloc(const FireSettings* settings, float 
     const int bx = nx <= 32 ? 32 : (nx <= 64 ? 64 : 128);
     const dim3 grid((nx + bx - 1) / bx, ny, nz);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // No lattice storage here: every curl-noise corner is hashed in place.
-    const firesim::HashLattice2 noLattice{};
-    firesim::forceContributions<<<grid, bx, 0, s>>>(scratch, in, vel, p, noLattice, noLattice);
+    // The curl noise's hashes: from lattices built for this call, as in a step,
+    // or in place (a null table) where the grid is small.
+    firesim::HashLattice2 curlA{}, curlB{};
+    if (cells >= kLatticeMinCells) {
+        int na = 0, nb = 0;
+        firesim::planCurlLattices(p.time, curlA, curlB, na, nb);
+        if (na <= firesim::kCurlLatticeEntries && nb <= firesim::kCurlLatticeEntries) {
+            curlA.values = lattice;
+            curlB.values = lattice + firesim::kCurlLatticeEntries;
+            firesim::hashLatticeBuild<<<dim3(256, 2), 256, 0, s>>>(curlA, curlB);
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return fail(std::string("force pass launch: ") + cudaGetErrorString(e));
+        }
+    }
+    firesim::forceContributions<<<grid, bx, 0, s>>>(scratch, in, vel, p, curlA, curlB);
     e = cudaGetLastError();  // nothing was pending on entry, so an error here is this launch's
     if (e != cudaSuccess) return fail(std::string("force pass launch: ") + cudaGetErrorString(e));
     firesim::forceProjectSetup<<<grid, bx, 0, s>>>(reinterpret_cast<firesim::FaceT*>(uOut), reinterpret_cast<firesim::FaceT*>(vOut),

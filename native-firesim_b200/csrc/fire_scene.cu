@@ -1026,10 +1026,15 @@ int planLattice(double pxLo, double pxHi, double pyLo, double pyHi, HashLattice2
 // The curl noise of forceContributions hashes, per cell at (u, v, w) in [0, 1]^3,
 //   A: (u * 9 + w * 3.7 + t * 0.22, v * 13 - t * 0.31)
 //   B: (w * 10 - t * 0.19, u * 8 + v * 5.5 + t * 0.27)        (src/fire_cuda.cu:1164-1165)
+void planCurlLattices(float time, HashLattice2& a, HashLattice2& b, int& na, int& nb) {
+    const double t = time;
+    na = planLattice(t * 0.22 - 1.0, 12.7 + t * 0.22 + 1.0, -t * 0.31 - 1.0, 13.0 - t * 0.31 + 1.0, a);
+    nb = planLattice(-t * 0.19 - 1.0, 10.0 - t * 0.19 + 1.0, t * 0.27 - 1.0, 13.5 + t * 0.27 + 1.0, b);
+}
+
 bool Scene::curlLattices(const FrameParams& p, HashLattice2& a, HashLattice2& b) const {
-    const double t = p.time;
-    const int na = planLattice(t * 0.22 - 1.0, 12.7 + t * 0.22 + 1.0, -t * 0.31 - 1.0, 13.0 - t * 0.31 + 1.0, a);
-    const int nb = planLattice(-t * 0.19 - 1.0, 10.0 - t * 0.19 + 1.0, t * 0.27 - 1.0, 13.5 + t * 0.27 + 1.0, b);
+    int na = 0, nb = 0;
+    planCurlLattices(p.time, a, b, na, nb);
     const bool fits = latticesEnabled_ && curlLattice_ != nullptr && static_cast<size_t>(na) <= curlCapacity_[0] &&
                       static_cast<size_t>(nb) <= curlCapacity_[1];
     a.values = fits ? curlLattice_ : nullptr;
