@@ -250,6 +250,15 @@ constexpr MgTile kMgTiles[kMgTileShapes] = {{32, 16, 16}, {16, 16, 8}, {16, 8, 8
 inline long long mgTiles(const MgTile& t, const MgLevel& L) {
     return static_cast<long long>((L.nx + t.x - 1) / t.x) * ((L.ny + t.y - 1) / t.y) * ((L.nz + t.z - 1) / t.z);
 }
+// Whether the smoothing's tiles interpolate from a coarse level (one that halves
+// every axis); otherwise the prolongation is a phase of its own.
+__host__ __device__ inline bool mgTileProlongs(const MgLevel& coarse) { return coarse.cx && coarse.cy && coarse.cz; }
+// Floats of shared memory of a tile: p and the rhs of its region and the coarse
+// cells it interpolates from.
+inline size_t mgTileFloats(const MgTile& t) {
+    const int x = t.x + 2 * kMgPassHalves, y = t.y + 2 * kMgPassHalves, z = t.z + 2 * kMgPassHalves;
+    return 2 * static_cast<size_t>(x) * y * z + static_cast<size_t>(x / 2 + 2) * (y / 2 + 2) * (z / 2 + 2);
+}
 inline int mgTileCells(const MgTile& t) { return (t.x + 2 * kMgPassHalves) * (t.y + 2 * kMgPassHalves) * (t.z + 2 * kMgPassHalves); }
 // Passes of a smoothing of `halves` half sweeps, and of the post-smoothing: the
 // passes of a cycle alternate between a level's two buffers, so their number is
@@ -275,9 +284,10 @@ struct MgScene {
 };
 // The work lists of a solve, as prefix sums over the scenes (0 for a scene
 // whose tail starts at or above the level).  tileUnits counts the smoothing's
-// tiles of grid level l, fineUnits the prolongation's units: where the row
-// length is a multiple of 4, 128 consecutive cells in memory, four per lane
-// (mgQuadUnits); otherwise 32-cell chunks of single rows.  coarseUnits counts the restriction's
+// tiles of grid level l, fineUnits the units of the prolongation phase (of the
+// scenes whose tiles do not interpolate): where the row length is a multiple of
+// 4, 128 consecutive cells in memory, four per lane (mgQuadUnits); otherwise
+// 32-cell chunks of single rows.  coarseUnits counts the restriction's
 // units of level l + 1: 64 consecutive coarse cells where the fine row length
 // is a multiple of 4, else 32-cell chunks of single rows.  chunks counts the
 // residual's chunks of level 0 (mgResidualChunks), allUnits the units of

@@ -31,10 +31,10 @@
 // CTAs are all co-resident (cooperative launch); the phases of a cycle are
 // separated by a grid barrier (a monotonic arrival count with release and
 // acquire semantics) whose waits are bounded in time.  A smoothing runs up to
-// four half sweeps per phase on tiles in shared memory, a CTA per tile; in the
-// other phases warps take the units of all scenes at that level from one work
-// list.  A level's
-// first colour-0 half sweep from p = 0 is written with its rhs (by the
+// four half sweeps per phase on tiles in shared memory, a CTA per tile, which
+// also interpolates the correction and averages the residual where it can; in
+// the other phases warps take the units of all scenes at that level from one
+// work list.  A level's first colour-0 half sweep from p = 0 is written with its rhs (by the
 // restriction, or the first phase for level 0 in the first cycle), as its
 // arithmetic reduces to (rhs + 0) / diag there.
 // The coarse end of each scene's hierarchy (from the first level of at most
@@ -228,7 +228,9 @@ __device__ __forceinline__ void tailSmoothLanes(float* __restrict__ p, const flo
 // goes to tailSmoothLanes; one of at most 128 cells is relaxed by the first
 // warp alone, with warp barriers; otherwise by the whole CTA.  skipFirst:
 // the first colour-0 half sweep was already done (from p = 0, by whoever
-// wrote the level's rhs).
+// wrote the level's rhs).  The loops are not unrolled: each level's smoothing is
+// code of its own, and by four its fetches cost more than the loads in flight
+// gave (a V-cycle 150 -> 147 us at 128^3, 155 -> 141 us at 200x24x216).
 template <bool PG, bool RG>
 __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* __restrict__ rhs, const MgLevel L, int sweeps,
                                            bool skipFirst) {
@@ -256,7 +258,7 @@ __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* _
             for (int s = 0; s < sweeps; ++s) {
                 for (int colour = skipFirst && s == 0 ? 1 : 0; colour < 2; ++colour) {
                     if (m.active) {
-#pragma unroll 4
+#pragma unroll 1
                         for (int z = z0 ^ colour; z < L.nz; z += dz) {
                             const int i = m.col + z * cols;
                             p[i] = weightedSum(load, tailLoad<RG>(rhs, i), L, i, x, y, z, load(i)) * L.invDiag;
@@ -270,7 +272,7 @@ __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* _
                 for (int colour = skipFirst && s == 0 ? 1 : 0; colour < 2; ++colour) {
                     for (int col = m.col; col < cols; col += m.colStride) {
                         const int y = col / L.nx, x = col - y * L.nx;
-#pragma unroll 4
+#pragma unroll 1
                         for (int z = (colour + x + y) & 1; z < L.nz; z += 2) {
                             const int i = col + z * cols;
                             p[i] = weightedSum(load, tailLoad<RG>(rhs, i), L, i, x, y, z, load(i)) * L.invDiag;
@@ -520,6 +522,18 @@ __device__ __forceinline__ float quadSum(const MgLevel& L, const Quad& q, int e,
 // wavefront) and 0.7 us to store.  A V-cycle went 208 -> 169 us at 128^3, 711 ->
 // 671 us at 256^3 and 119 -> 93 us at 64^3.
 //
+// The transfers between levels run on the loaded tiles too: the correction is
+// interpolated into the tile before the post-smoothing (2 us a tile of 32x16x16,
+// where a phase over global memory took 12 us at 128^3, 75 us at 256^3, 4.5 us
+// at 32^3, 2 us of it barrier), the residual averaged from it after a
+// pre-smoothing whose last pass leaves the cells beside the tile valid (1.9 us a
+// tile; 8, 50 and 4.5 us).  With it a thread that has no column prepares the next
+// tile's operands.  A V-cycle went 169 -> 147 us at 128^3, 671 -> 635 us at 256^3
+// and 93 -> 80 us at 64^3.  The tile's stages are functions of their own: inlined
+// into one, or with the load and the interpolation in one, they spill, and a
+// cycle takes 160-240 us at 128^3; the phases over global memory, the other way
+// round, are slower as functions (175 us).
+//
 // A CTA loads a tile of p and the rhs with a halo of four cells, runs `count`
 // half sweeps on it (each valid one cell less far into the halo) and writes the
 // tile's own cells to the level's other buffer, so that neighbouring tiles
@@ -543,7 +557,9 @@ struct TileShape {
     static constexpr int PLANE = RY * K, COLOUR = RZ * PLANE;
     static constexpr int COLS = RY * QUADS;
     static constexpr int GROUPS = kMgThreads / COLS;
-    static constexpr int LOADS = QUADS * RY * RZ;
+    static constexpr int PER = (RZ + GROUPS - 1) / GROUPS;  // planes that a group loads
+    // The coarse cells that the region interpolates from, where every axis is halved.
+    static constexpr int CX = (TX + 2 * H) / 2 + 2, CY = RY / 2 + 2, CZ = RZ / 2 + 2;
     static_assert(GROUPS >= 1 && 2 * COLOUR == (TX + 2 * H) * RY * RZ, "tile shape");
 };
 
@@ -620,60 +636,287 @@ __device__ __forceinline__ void tileHalfSweep(const MgLevel& L, float* smem, int
     }
 }
 
+// One tile's share of a smoothing pass: half sweeps first .. first + count - 1
+// from src to dst; before them, where correction is set, the interpolated
+// correction of the coarse level is added to p; after them, where coarseRhs is
+// set (count at most 3, so that the cells beside the tile are valid too), the
+// residual is averaged onto the coarse level, whose p becomes zero or, with red,
+// its first colour-0 half sweep.
+struct TileJob {
+    MgLevel L, C;  // the level and the coarse level
+    const float *src, *rhs;
+    float* dst;
+    const float* correction;
+    float *coarseRhs, *coarseP;
+    int unit, red, x0, y0, z0;
+};
+// The CTA's tile and the next one, in shared memory: operands that the stages
+// below read from there cost no registers, and a thread without cells prepares
+// the next tile while the others smooth (0.9 us of latency a tile else).
+__shared__ TileJob sTile[2];
+
+// The residuals of the cells x (even) and x + 1 of row (y, z), both in slot k.
 template <int TX, int TY, int TZ>
-__device__ __noinline__ void tileSmooth(const MgLevel& level, const float* __restrict__ src, const float* __restrict__ rhs,
-                                        float* __restrict__ dst, int tile, int first, int count) {
+__device__ __forceinline__ float2 tileResidual(const MgLevel& L, const float* smem, int at, int x, int y, int z) {
     using S = TileShape<TX, TY, TZ>;
-    extern __shared__ float smem[];  // [p, rhs][colour][RZ][RY][K]
-    const MgLevel L = level;
-    const int tilesX = (L.nx + TX - 1) / TX, tilesY = (L.ny + TY - 1) / TY;
-    const int tz = tile / (tilesX * tilesY), ty = (tile - tz * tilesX * tilesY) / tilesX, tx = tile - (tz * tilesY + ty) * tilesX;
-    const int x0 = tx * TX, y0 = ty * TY, z0 = tz * TZ;
-    const bool whole = (L.nx & 3) == 0;
-    constexpr int BATCH = 3;  // quads in flight per thread
+    // Even cells of the row have colour (y + z) & 1; rows beside it the other.
+    const int even = (y + z) & 1;
+    const float* e = smem + even * S::COLOUR + at;
+    const float* o = smem + (1 - even) * S::COLOUR + at;
+    const float ec = e[0], oc = o[0];
+    const float eL = x > 0 ? o[-1] : ec, eR = x < L.nx - 1 ? oc : ec;
+    const float oL = ec, oR = x + 1 < L.nx - 1 ? e[1] : oc;
+    const float eD = y > 0 ? o[-S::K] : ec, oD = y > 0 ? e[-S::K] : oc;
+    const float eU = y < L.ny - 1 ? o[S::K] : 0.0f - ec, oU = y < L.ny - 1 ? e[S::K] : 0.0f - oc;
+    const float eB = z > 0 ? o[-S::PLANE] : ec, oB = z > 0 ? e[-S::PLANE] : oc;
+    const float eF = z < L.nz - 1 ? o[S::PLANE] : ec, oF = z < L.nz - 1 ? e[S::PLANE] : oc;
+    return make_float2(combine(e[2 * S::COLOUR], eL, eR, eD, eU, eB, eF, L) - L.diag * ec,
+                       combine(o[2 * S::COLOUR], oL, oR, oD, oU, oB, oF, L) - L.diag * oc);
+}
+
+// The tile's coarse cells: restrictAt from shared memory.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void tileRestrict(int buf) {
+    using S = TileShape<TX, TY, TZ>;
+    extern __shared__ float smem[];
+    const TileJob& job = sTile[buf];
+    const MgLevel L = job.L, C = job.C;
+    const int x0 = job.x0, y0 = job.y0, z0 = job.z0;
+    auto put = [&](int X, int Y, int Z, float r) {
+        const int c = mgAt(C, X, Y, Z);
+        job.coarseRhs[c] = r;
+        job.coarseP[c] = job.red && ((X + Y + Z) & 1) == 0 ? (r + 0.0f) * C.invDiag : 0.0f;
+    };
+    if (mgTileProlongs(C)) {
+        // Every axis halved: the eight fine cells share their neighbours, which
+        // are loaded whether or not a wall takes their place (the halo is there).
+        for (int i = threadIdx.x; i < TX / 2 * (TY / 2) * (TZ / 2); i += kMgThreads) {
+            const int row = i / (TX / 2), a = i - row * (TX / 2);
+            const int d = row / (TY / 2), b = row - d * (TY / 2);
+            const int x = x0 + 2 * a, y = y0 + 2 * b, z = z0 + 2 * d;
+            if (x >= L.nx || y >= L.ny || z >= L.nz) continue;
+            const float* at = smem + ((z - z0 + S::H) * S::RY + (y - y0 + S::H)) * S::K + ((x - x0 + S::H) >> 1);
+            // The even and the odd cell of row (dy, dz): x, y and z are even.
+            auto even = [&](int dy, int dz) { return at[((dy + dz) & 1) * S::COLOUR + dz * S::PLANE + dy * S::K]; };
+            auto odd = [&](int dy, int dz) { return at[((dy + dz + 1) & 1) * S::COLOUR + dz * S::PLANE + dy * S::K]; };
+            float plane[2];
+#pragma unroll
+            for (int dz = 0; dz < 2; ++dz) {
+                float mean[2];
+#pragma unroll
+                for (int dy = 0; dy < 2; ++dy) {
+                    const int ce = ((dy + dz) & 1) * S::COLOUR + dz * S::PLANE + dy * S::K;
+                    const int co = ((dy + dz + 1) & 1) * S::COLOUR + dz * S::PLANE + dy * S::K;
+                    const float e = even(dy, dz), o = odd(dy, dz);
+                    const float before = at[co - 1], after = at[ce + 1];
+                    const float eL = x > 0 ? before : e, oR = x + 1 < L.nx - 1 ? after : o;
+                    const bool low = dy == 0 && y == 0, back = dz == 0 && z == 0;
+                    const bool high = dy == 1 && y + 1 == L.ny - 1, front = dz == 1 && z + 1 == L.nz - 1;
+                    const float eD = even(dy - 1, dz), oD = odd(dy - 1, dz), eU = even(dy + 1, dz), oU = odd(dy + 1, dz);
+                    const float eB = even(dy, dz - 1), oB = odd(dy, dz - 1), eF = even(dy, dz + 1), oF = odd(dy, dz + 1);
+                    const float re = combine(at[ce + 2 * S::COLOUR], eL, o, low ? e : eD, high ? 0.0f - e : eU, back ? e : eB, front ? e : eF, L) - L.diag * e;
+                    const float ro = combine(at[co + 2 * S::COLOUR], e, oR, low ? o : oD, high ? 0.0f - o : oU, back ? o : oB, front ? o : oF, L) - L.diag * o;
+                    mean[dy] = 0.5f * (re + ro);
+                }
+                plane[dz] = 0.5f * (mean[0] + mean[1]);
+            }
+            put(x >> 1, y >> 1, z >> 1, 0.5f * (plane[0] + plane[1]));
+        }
+        return;
+    }
+    const int cw = C.cx ? TX / 2 : TX, ch = C.cy ? TY / 2 : TY, cd = C.cz ? TZ / 2 : TZ;
+    for (int i = threadIdx.x; i < cw * ch * cd; i += kMgThreads) {
+        const int row = i / cw, a = i - row * cw;
+        const int d = row / ch, b = row - d * ch;
+        const int x = x0 + (C.cx ? 2 * a : a), y = y0 + (C.cy ? 2 * b : b), z = z0 + (C.cz ? 2 * d : d);
+        if (x >= L.nx || y >= L.ny || z >= L.nz) continue;
+        const int at = ((z - z0 + S::H) * S::RY + (y - y0 + S::H)) * S::K + ((x - x0 + S::H) >> 1);
+        float plane[2] = {0.0f, 0.0f};
 #pragma unroll 1
-    for (int i0 = threadIdx.x; i0 < S::LOADS; i0 += BATCH * kMgThreads) {
+        for (int dz = 0; dz <= C.cz; ++dz) {
+            float mean[2] = {0.0f, 0.0f};
+#pragma unroll 1
+            for (int dy = 0; dy <= C.cy; ++dy) {
+                const float2 r = tileResidual<TX, TY, TZ>(L, smem, at + dz * S::PLANE + dy * S::K, x & ~1, y + dy, z + dz);
+                const float m = C.cx ? 0.5f * (r.x + r.y) : ((x & 1) != 0 ? r.y : r.x);
+                if (dy == 0) mean[0] = m; else mean[1] = m;
+            }
+            const float m = C.cy ? 0.5f * (mean[0] + mean[1]) : mean[0];
+            if (dz == 0) plane[0] = m; else plane[1] = m;
+        }
+        put(C.cx ? x >> 1 : x, C.cy ? y >> 1 : y, C.cz ? z >> 1 : z, C.cz ? 0.5f * (plane[0] + plane[1]) : plane[0]);
+    }
+}
+
+// The coarse plane Z interpolated along x and y to the four cells of the
+// region's quad q of row ly, from the coarse cells in shared memory (every axis
+// halved; cells past the level's ends hold the clamped neighbour): prolongAt's
+// weights and order.
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ float4 tileProlong(const float* coarse, int q, int ly, int Z) {
+    using S = TileShape<TX, TY, TZ>;
+    const int Y0 = (ly >> 1) + 1, Y1 = (ly & 1) ? Y0 + 1 : Y0 - 1;
+    const float* near = coarse + (Z * S::CY + Y0) * S::CX + 2 * q;  // coarse x b - 1, b | b + 1, b + 2
+    const float* far = coarse + (Z * S::CY + Y1) * S::CX + 2 * q;
+    const float2 u = at2(near), v = at2(near + 2), s = at2(far), t = at2(far + 2);
+    auto blend = [](float a, float b) { return 0.75f * a + 0.25f * b; };
+    return make_float4(blend(blend(u.y, u.x), blend(s.y, s.x)), blend(blend(u.y, v.x), blend(s.y, t.x)),
+                       blend(blend(v.x, u.y), blend(t.x, s.y)), blend(blend(v.x, v.y), blend(t.x, t.y)));
+}
+
+// Loads the tile with its halo, and the coarse cells beside it where a
+// correction follows.  Slots outside the grid keep what they hold.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void tileLoad(int buf) {
+    using S = TileShape<TX, TY, TZ>;
+    extern __shared__ float smem[];  // [p, rhs][colour][RZ][RY][K], then the coarse cells [CZ][CY][CX]
+    const TileJob& job = sTile[buf];
+    const int x0 = job.x0, y0 = job.y0, z0 = job.z0;
+    const float* correction = job.correction;
+    if (correction != nullptr) {
+        const int cx = job.C.nx, cy = job.C.ny, cz = job.C.nz;
+        float* coarse = smem + 4 * S::COLOUR;
+        for (int i = threadIdx.x; i < S::CX * S::CY * S::CZ; i += kMgThreads) {
+            const int row = i / S::CX, a = i - row * S::CX;
+            const int d = row / S::CY, b = row - d * S::CY;
+            const int X = min(max((x0 - S::H) / 2 - 1 + a, 0), cx - 1);
+            const int Y = min(max((y0 - S::H) / 2 - 1 + b, 0), cy - 1);
+            const int Z = min(max((z0 - S::H) / 2 - 1 + d, 0), cz - 1);
+            const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(coarse + i));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(correction + (Z * cy + Y) * cx + X) : "memory");
+        }
+    }
+    // A thread loads the quad q of row ly in the planes of its group.
+    const int nx = job.L.nx, ny = job.L.ny, nz = job.L.nz;
+    const int group = threadIdx.x / S::COLS, col = threadIdx.x - group * S::COLS;
+    const int ly = col / S::QUADS, q = col - ly * S::QUADS;
+    const int x = x0 - S::H + 4 * q, y = y0 - S::H + ly;
+    const bool in = x >= 0 && x < nx && y >= 0 && y < ny;
+    const int lzA = max(group * S::PER, S::H - z0), lzB = in ? min(min(group * S::PER + S::PER, S::RZ), nz - z0 + S::H) : 0;
+    const int plane = nx * ny, n = nx - x;
+    const bool whole = (nx & 3) == 0;
+    int g = ((z0 - S::H + lzA) * ny + y) * nx + x;
+    constexpr int BATCH = S::PER < 3 ? S::PER : 3;  // quads in flight per thread
+#pragma unroll 1
+    for (int lz0 = lzA; lz0 < lzB; lz0 += BATCH, g += BATCH * plane) {
         float4 p[BATCH], r[BATCH];
+        const float* src = job.src + g;
+        const float* rhs = job.rhs + g;
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
-            const int i = i0 + j * kMgThreads;
-            const int row = i / S::QUADS, q = i - row * S::QUADS;
-            const int lz = row / S::RY, ly = row - lz * S::RY;
-            const int x = x0 - S::H + 4 * q, y = y0 - S::H + ly, z = z0 - S::H + lz;
-            const bool in = i < S::LOADS && x >= 0 && x < L.nx && y >= 0 && y < L.ny && z >= 0 && z < L.nz;
-            const int g = (z * L.ny + y) * L.nx + x;
             p[j] = r[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (in && whole) {
-                p[j] = ldcg4(src + g);
-                r[j] = ldcg4(rhs + g);
-            } else if (in) {
-                const float* a = src + g;
-                const float* b = rhs + g;
-                const int n = L.nx - x;
+            if (lz0 + j >= lzB) continue;
+            if (whole) {
+                p[j] = ldcg4(src + j * plane);
+                r[j] = ldcg4(rhs + j * plane);
+            } else {
+                const float* a = src + j * plane;
+                const float* b = rhs + j * plane;
                 p[j] = make_float4(__ldcg(a), n > 1 ? __ldcg(a + 1) : 0.0f, n > 2 ? __ldcg(a + 2) : 0.0f, n > 3 ? __ldcg(a + 3) : 0.0f);
                 r[j] = make_float4(__ldcg(b), n > 1 ? __ldcg(b + 1) : 0.0f, n > 2 ? __ldcg(b + 2) : 0.0f, n > 3 ? __ldcg(b + 3) : 0.0f);
             }
         }
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
-            const int i = i0 + j * kMgThreads;
-            if (i >= S::LOADS) break;
-            const int row = i / S::QUADS, q = i - row * S::QUADS;
-            const int lz = row / S::RY, ly = row - lz * S::RY;
-            const int even = (y0 + ly + z0 + lz) & 1;  // the colour of the row's even cells (the halo is even)
-            float* e = smem + even * S::COLOUR + row * S::K + 2 * q;
-            float* o = smem + (1 - even) * S::COLOUR + row * S::K + 2 * q;
+            const int lz = lz0 + j;
+            if (lz >= lzB) break;
+            const int even = (ly + lz) & 1;  // the colour of the row's even cells (tiles and the halo are even)
+            const int at = (lz * S::RY + ly) * S::K + 2 * q;
+            float* e = smem + even * S::COLOUR + at;
+            float* o = smem + (1 - even) * S::COLOUR + at;
             *reinterpret_cast<float2*>(e) = make_float2(p[j].x, p[j].z);
             *reinterpret_cast<float2*>(o) = make_float2(p[j].y, p[j].w);
             *reinterpret_cast<float2*>(e + 2 * S::COLOUR) = make_float2(r[j].x, r[j].z);
             *reinterpret_cast<float2*>(o + 2 * S::COLOUR) = make_float2(r[j].y, r[j].w);
         }
     }
+    if (correction != nullptr) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+}
+
+// p += the coarse correction in the loaded tile and its halo.  A thread walks
+// its quad along z with the coarse planes behind and at it interpolated along x
+// and y, so that each is interpolated once for two planes.  Slots outside the
+// grid get values that no valid cell reads.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void tileCorrect() {
+    using S = TileShape<TX, TY, TZ>;
+    extern __shared__ float smem[];
+    const float* coarse = smem + 4 * S::COLOUR;
+    const int group = threadIdx.x / S::COLS, col = threadIdx.x - group * S::COLS;
+    const int ly = col / S::QUADS, q = col - ly * S::QUADS;
+    constexpr int PER = (S::RZ / 2 + S::GROUPS - 1) / S::GROUPS * 2;  // an even number of planes a thread
+    const int lzA = group * PER, lzB = min(lzA + PER, S::RZ);
+    if (lzA < lzB) {
+        float4 behind = tileProlong<TX, TY, TZ>(coarse, q, ly, lzA / 2), at = tileProlong<TX, TY, TZ>(coarse, q, ly, lzA / 2 + 1);
+        auto add = [&](int lz, const float4& other) {
+            const int even = (ly + lz) & 1;
+            const int i = (lz * S::RY + ly) * S::K + 2 * q;
+            float2* e = reinterpret_cast<float2*>(smem + even * S::COLOUR + i);
+            float2* o = reinterpret_cast<float2*>(smem + (1 - even) * S::COLOUR + i);
+            const float2 a = *e, b = *o;
+            *e = make_float2(a.x + (0.75f * at.x + 0.25f * other.x), a.y + (0.75f * at.z + 0.25f * other.z));
+            *o = make_float2(b.x + (0.75f * at.y + 0.25f * other.y), b.y + (0.75f * at.w + 0.25f * other.w));
+        };
+#pragma unroll 1
+        for (int lz = lzA; lz < lzB; lz += 2) {
+            const float4 front = tileProlong<TX, TY, TZ>(coarse, q, ly, lz / 2 + 2);
+            add(lz, behind);
+            add(lz + 1, front);
+            behind = at;
+            at = front;
+        }
+    }
+    __syncthreads();
+}
+
+// The next tile's rows into L2, by the warps that have no columns, where the
+// level's p, its other buffer and its rhs exceed the L2: a V-cycle at 256^3
+// (201 MB) went 666 -> 647 us.  At 192^3 (85 MB), where the rows are in L2, it
+// went 317 -> 320 us, at 128^3 148 -> 151.
+constexpr int kMgL2Cells = (126 << 20) / 12;
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ void tilePrefetch(int buf, int total) {
+    using S = TileShape<TX, TY, TZ>;
+    constexpr int kFirst = S::GROUPS * S::COLS / 32 * 32 < kMgThreads - 32 ? S::GROUPS * S::COLS / 32 * 32 : kMgThreads - 32;
+    if (threadIdx.x < kFirst) return;
+    __syncwarp();
+    const TileJob& job = sTile[buf];
+    if (job.unit >= total) return;
+    const int nx = job.L.nx, ny = job.L.ny, nz = job.L.nz;
+    const int x = max(job.x0 - S::H, 0);
+    for (int i = threadIdx.x - kFirst; i < S::RY * S::RZ; i += kMgThreads - kFirst) {
+        const int lz = i / S::RY, y = job.y0 - S::H + i - lz * S::RY, z = job.z0 - S::H + lz;
+        if (y < 0 || y >= ny || z < 0 || z >= nz) continue;
+        const int g = (z * ny + y) * nx;
+        const int last = min(job.x0 + TX + S::H, nx) - 1;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + x));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + x));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + last));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + last));
+    }
+}
+
+// Half sweeps first .. first + count - 1 of the loaded tile, its restriction and
+// its store.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void tileSmooth(int buf, int first, int count, int total) {
+    using S = TileShape<TX, TY, TZ>;
+    extern __shared__ float smem[];
+    const TileJob& job = sTile[buf];
+    const MgLevel L = job.L;
+    const int x0 = job.x0, y0 = job.y0, z0 = job.z0;
+    // With the restriction the cells beside the tile stay valid to the end.
+    const int beyond = job.coarseRhs != nullptr ? 1 : 0;
+    if (job.correction != nullptr) tileCorrect<TX, TY, TZ>();
+    if (L.nx * L.ny * L.nz > kMgL2Cells) tilePrefetch<TX, TY, TZ>(buf ^ 1, total);
     for (int s = 0; s < count; ++s) {
-        tileHalfSweep<TX, TY, TZ>(L, smem, x0, y0, z0, (first + s) & 1, count - 1 - s);
+        tileHalfSweep<TX, TY, TZ>(L, smem, x0, y0, z0, (first + s) & 1, count - 1 - s + beyond);
         __syncthreads();
     }
+    if (beyond != 0) tileRestrict<TX, TY, TZ>(buf);
+    const bool whole = (L.nx & 3) == 0;
+    float* __restrict__ dst = job.dst;
     for (int i = threadIdx.x; i < TX / 4 * TY * TZ; i += kMgThreads) {
         const int row = i / (TX / 4), q = i - row * (TX / 4);
         const int lz = row / TY, ly = row - lz * TY;
@@ -739,43 +982,92 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     }
     __syncthreads();
     auto converged = [&](int s) { return sRunning[s] == 0; };
+    const bool redFirst = pre > 0;
+    const int prePasses = mgSmoothPasses(2 * pre), postPasses = mgPostPasses(pre, post);
     // Half sweeps first .. first + count - 1 (count <= kMgPassHalves) of level l
     // of every scene that has it as a grid level, one tile per CTA at a time.
     // The results go to the level's other buffer (side: 0 if they come from p).
-    auto smooth = [&](int l, int first, int count, int side) {
+    // prolong: the coarse correction is added first, where every axis is halved
+    // (else prolongFrom has added it: a kept axis would need other weights and a
+    // coarse region of another shape); restrict: the restriction follows.
+    auto smooth = [&](int l, int first, int count, int side, bool prolong, bool restrict) {
         const int* off = plan->tileUnits[l];
         const int total = __ldg(off + n);
         const int shape = __ldg(&plan->tile[l]);
-        for (int unit = blockIdx.x; unit < total; unit += gridDim.x) {
-            const int s = sceneOf(off, n, unit);
-            if (converged(s)) continue;
+        // Fills sTile[buf] with the next tile at or after `unit` of a scene
+        // that still runs (unit: at least total if there is none).
+        auto prepare = [&](int buf, int unit) {
+            TileJob& job = sTile[buf];
+            int s = 0;
+            for (; unit < total; unit += gridDim.x) {
+                s = sceneOf(off, n, unit);
+                if (!converged(s)) break;
+            }
+            job.unit = unit;
+            if (unit >= total) return;
             const MgScene& S = scenes[s];
+            const MgLevel L = S.lv[l], C = S.lv[l + 1];
+            job.L = L;
+            job.C = C;
+            job.src = side ? S.q[l] : S.p[l];
+            job.dst = side ? S.p[l] : S.q[l];
+            job.rhs = S.rhs[l];
+            job.correction = prolong && mgTileProlongs(C) ? S.p[l + 1] : nullptr;
+            job.coarseRhs = restrict ? S.rhs[l + 1] : nullptr;
+            job.coarseP = S.p[l + 1];
+            job.red = redFirst && l + 1 < S.tail ? 1 : 0;
+            const int tx = shape == 0 ? kMgTiles[0].x : shape == 1 ? kMgTiles[1].x : shape == 2 ? kMgTiles[2].x : kMgTiles[3].x;
+            const int ty = shape == 0 ? kMgTiles[0].y : shape == 1 ? kMgTiles[1].y : shape == 2 ? kMgTiles[2].y : kMgTiles[3].y;
+            const int tz = shape == 0 ? kMgTiles[0].z : shape == 1 ? kMgTiles[1].z : shape == 2 ? kMgTiles[2].z : kMgTiles[3].z;
             const int tile = unit - __ldg(off + s);
-            const float* src = side ? S.q[l] : S.p[l];
-            float* dst = side ? S.p[l] : S.q[l];
+            const int tilesX = (L.nx + tx - 1) / tx, tilesY = (L.ny + ty - 1) / ty;
+            const int row = tile / tilesX, slice = row / tilesY;
+            job.x0 = (tile - row * tilesX) * tx;
+            job.y0 = (row - slice * tilesY) * ty;
+            job.z0 = slice * tz;
+        };
+        constexpr int kPreparer = kMgThreads - 1;
+        if (threadIdx.x == kPreparer) prepare(0, blockIdx.x);
+        __syncthreads();
+        for (int buf = 0; sTile[buf].unit < total; buf ^= 1) {
             if (shape == 0) {
-                tileSmooth<32, 16, 16>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+                tileLoad<32, 16, 16>(buf);
             } else if (shape == 1) {
-                tileSmooth<16, 16, 8>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+                tileLoad<16, 16, 8>(buf);
             } else if (shape == 2) {
-                tileSmooth<16, 8, 8>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+                tileLoad<16, 8, 8>(buf);
             } else {
-                tileSmooth<8, 8, 4>(S.lv[l], src, S.rhs[l], dst, tile, first, count);
+                tileLoad<8, 8, 4>(buf);
+            }
+            if (threadIdx.x == kPreparer) prepare(buf ^ 1, sTile[buf].unit + gridDim.x);
+            if (shape == 0) {
+                tileSmooth<32, 16, 16>(buf, first, count, total);
+            } else if (shape == 1) {
+                tileSmooth<16, 16, 8>(buf, first, count, total);
+            } else if (shape == 2) {
+                tileSmooth<16, 8, 8>(buf, first, count, total);
+            } else {
+                tileSmooth<8, 8, 4>(buf, first, count, total);
             }
         }
     };
     // A smoothing of `halves` half sweeps from half sweep `first` on, in
-    // `passes` passes of about equal length.
-    auto smoothLevel = [&](int l, int first, int halves, int passes, int& side) {
+    // `passes` passes of about equal length; false if a barrier failed.
+    // restricted: the last pass also restricts (it can where it is not full).
+    auto smoothLevel = [&](int l, int first, int halves, int passes, int& side, bool prolong, bool& restricted) {
         for (int k = 0; k < passes; ++k) {
             const int from = halves * k / passes, to = halves * (k + 1) / passes;
-            smooth(l, first + from, to - from, side);
+            const bool restrict = restricted && k + 1 == passes && to - from < kMgPassHalves;
+            if (k + 1 == passes) restricted = restrict;
+            smooth(l, first + from, to - from, side, prolong && k == 0, restrict);
             side ^= 1;
             if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return false;
         }
         return true;
     };
-    // Coarse rhs = the mean residual of the covered fine cells, and coarse p
+    // For the levels whose tiles do not restrict (a last pass of four half
+    // sweeps, as level 0's from the second cycle on with two sweeps):
+    // coarse rhs = the mean residual of the covered fine cells, and coarse p
     // = 0, or, when `red` (the coarse level is a grid level whose
     // pre-smoothing starts with the colour-0 half sweep), that half sweep's
     // result from p = 0: (rhs + 0) / diag on colour-0 cells (every neighbour
@@ -846,7 +1138,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             }
         }
     };
-    // p += the interpolated coarse correction.  Where the fine row length is
+    // For the scenes whose tiles do not interpolate (an axis is kept): p += the
+    // interpolated coarse correction.  Where the fine row length is
     // a multiple of 4, units are 128 consecutive fine cells in memory, a quad
     // per lane: for each of the four coarse rows the quad interpolates from,
     // the lane loads the coarse values at x0/2 and x0/2 + 1 and takes those
@@ -934,8 +1227,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
     // first cycle's colour-0 half sweep of level 0 is done here, as in
     // restrictTo: (rhs + 0) / diag on colour-0 cells, 0 elsewhere (scenes
     // whose level 0 is in the tail start from 0).  Units as the smoothing's.
-    const bool redFirst = pre > 0;
-    const int prePasses = mgSmoothPasses(2 * pre), postPasses = mgPostPasses(pre, post);
     {
         const int total = __ldg(plan->allUnits + n);
         for (int unit = gwarp; unit < total; unit += nwarps) {
@@ -985,9 +1276,12 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             // first cycle, was done with the restriction (the initialisation).
             const int done = redFirst && (l > 0 || cycle == 0) ? 1 : 0;
             int side = 0;
-            if (!smoothLevel(l, done, 2 * pre - done, prePasses, side)) return;
-            restrictTo(l, redFirst, side);
-            if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
+            bool restricted = true;
+            if (!smoothLevel(l, done, 2 * pre - done, prePasses, side, false, restricted)) return;
+            if (!restricted) {
+                restrictTo(l, redFirst, side);
+                if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
+            }
         }
         for (int s = blockIdx.x; s < n; s += gridDim.x) {
             if (!converged(s)) {
@@ -1005,9 +1299,12 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
         if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
         for (int l = gridLevels - 1; l >= 0; --l) {
             int side = prePasses & 1;
-            prolongFrom(l, side);
-            if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
-            if (!smoothLevel(l, 0, 2 * post, postPasses, side)) return;
+            if (__ldg(plan->fineUnits[l] + n) > 0) {
+                prolongFrom(l, side);
+                if (!gridBarrier(sync, generation, waitNs, hostStatus, ++phase)) return;
+            }
+            bool restricted = false;
+            if (!smoothLevel(l, 0, 2 * post, postPasses, side, true, restricted)) return;
         }
         if (gated) {
             // Level-0 residual, one warp per chunk (mgResidualChunk: a fixed

@@ -843,7 +843,7 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
         for (int s = 0; s < n; ++s) {
             plan.tileUnits[l][s + 1] = plan.tileUnits[l][s] + (l < scenes[s].tail ? static_cast<int>(mgTiles(t, scenes[s].lv[l])) : 0);
         }
-        smem = std::max(smem, 2 * sizeof(float) * static_cast<size_t>(mgTileCells(t)));
+        smem = std::max(smem, sizeof(float) * mgTileFloats(t));
     }
     std::memcpy(hScenes, scenes.data(), n * sizeof(MgScene));
     int perSm = 0;
@@ -859,7 +859,7 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
             const MgLevel& F = S.lv[l];
             const bool quad = (F.nx & 3) == 0;
             const int fine = quad ? mgQuadUnits(F.nx, F.ny, F.nz) : F.ny * F.nz * mgRowChunks(F.nx);
-            plan.fineUnits[l][s + 1] = plan.fineUnits[l][s] + (grid ? fine : 0);
+            plan.fineUnits[l][s + 1] = plan.fineUnits[l][s] + (grid && !mgTileProlongs(S.lv[l + 1]) ? fine : 0);
             if (grid) {
                 const MgLevel& C = S.lv[l + 1];
                 const int coarse = quad ? (C.nx * C.ny * C.nz + 63) / 64 : C.ny * C.nz * mgRowChunks(C.nx);
