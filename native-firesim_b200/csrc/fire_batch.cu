@@ -176,6 +176,7 @@ bool BatchRunner::run(const FireSettings* settings, const int* render, std::stri
     ++launched;
     go(batchSubtractIncrement, kBatchCells);
     if (anyRender) {
+        go(batchOccupancy, kBatchBricks);
         go(batchTransmittance, kBatchLight);
         go(batchRaymarch, kBatchPixels);
         go(batchPackHdr, kBatchPixels);

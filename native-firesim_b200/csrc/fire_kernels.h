@@ -211,8 +211,33 @@ __global__ void cfgVorticity(float4* vort, Velocity vel, ConfigParams p);
 __global__ void cfgNoiseField(float4* noise, ConfigParams p);
 __global__ void cfgCellForce(float4* force, const float4* vort, const Rec4* a, const float4* noise, ConfigParams p);
 __global__ void cfgApplyForces(FaceT* uOut, FaceT* vOut, FaceT* wOut, Velocity vel, const float4* force, ConfigParams p);
-__global__ void cfgTransmittance(float* tr, const Rec4* a, ConfigParams p);
-__global__ void cfgRaymarch(float4* hdr, const Rec4* a, const float* tr, ConfigParams p);
+// Which bricks of 4x4x4 cells a trilinear sample of record a can see something
+// in: a brick's flag (a byte each, x fastest, after the header) is set if heat,
+// fuel or soot is not zero in any cell that a sample whose first corner lies in
+// the brick reads.  box is the bounding box of the set bricks: 2^20 - lo and
+// hi + 1 per axis, so that zero is empty.  irregular: some transmittance is not
+// within +-1e30, so that a sample of nothing need not add nothing.  dense: half
+// of the bricks or more are set.  done and the acc fields are the build's own,
+// zero between builds.
+struct CfgOccupancy {
+    unsigned done, accIrregular, irregular, accSet, dense, unused[3];
+    unsigned acc[6], box[6];
+};
+__host__ __device__ inline int cfgBricks(int n) { return (n + 3) >> 2; }
+inline size_t cfgOccupancyBytes(int nx, int ny, int nz) {
+    return sizeof(CfgOccupancy) + static_cast<size_t>(cfgBricks(nx)) * cfgBricks(ny) * cfgBricks(nz);
+}
+// A warp builds seven bricks along x (lane 28 reads the cells that the last one
+// shares with the next).
+__host__ __device__ inline int cfgOccupancyUnits(int nx, int ny, int nz) {
+    return ((cfgBricks(nx) + 6) / 7) * cfgBricks(ny) * cfgBricks(nz);
+}
+__global__ void cfgOccupancyBuild(CfgOccupancy* occ, const Rec4* a, const float* tr, ConfigParams p);
+constexpr int kRayLanes = 4;  // lanes of a ray in the Lanes kernels
+__global__ void cfgTransmittance(float* tr, const Rec4* a, CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgTransmittanceLanes(float* tr, const Rec4* a, CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgRaymarchLanes(float4* hdr, const Rec4* a, const float* tr, const CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgRaymarch(float4* hdr, const Rec4* a, const float* tr, const CfgOccupancy* occ, ConfigParams p);
 
 // ---------------------------------------------------------------------------
 // Multigrid pressure solve of the config physics (fire_mg.cu): the
@@ -334,10 +359,10 @@ __global__ void cfgTopFaces(FaceT* v, const float* p, int nx, int ny, int nz);
 // Batched config physics (fire_config.cu, host side fire_batch.cu): one launch
 // per stage over every scene of a batch.  A block belongs to one scene; its
 // threads take consecutive elements of one index space of that scene (x
-// fastest): cells, faces ((nx+1)(ny+1)(nz+1)), half-resolution light cells
-// or pixels.  The per-element work is the single-scene kernels' own body, so
+// fastest): cells, faces ((nx+1)(ny+1)(nz+1)), half-resolution light cells,
+// pixels, or the lanes of the occupancy's warps.  The per-element work is the single-scene kernels' own body, so
 // a scene gives the same bits alone or in a batch.
-enum BatchSpace { kBatchCells = 0, kBatchFaces = 1, kBatchLight = 2, kBatchPixels = 3, kBatchSpaces = 4 };
+enum BatchSpace { kBatchCells = 0, kBatchFaces = 1, kBatchLight = 2, kBatchPixels = 3, kBatchBricks = 4, kBatchSpaces = 5 };
 constexpr int kBatchThreads = 128;
 // Elements per thread of a batched stage: runs of consecutive cells or faces
 // (one scene lookup and one coordinate division per run); one light column or
@@ -359,6 +384,7 @@ struct BatchScene {
     float* divergence;
     float* delta;          // the multigrid's level-0 increment
     float* transmittance;
+    CfgOccupancy* occupancy;
     float4* hdr;
     void* slot;            // the scene's HDR output buffer (null: keep the frame in hdr)
     size_t slotPitch;
@@ -377,6 +403,7 @@ __global__ void batchCellForce(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchApplyForces(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchPrepareIncrement(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchSubtractIncrement(const BatchScene* scenes, const BatchPlan* plan);
+__global__ void batchOccupancy(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchTransmittance(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchRaymarch(const BatchScene* scenes, const BatchPlan* plan);
 __global__ void batchPackHdr(const BatchScene* scenes, const BatchPlan* plan);

@@ -126,6 +126,7 @@ void Scene::release() {
     splitDiv_ = nullptr;
     cfgVort_ = nullptr;
     cfgLight_ = nullptr;
+    cfgOcc_ = nullptr;
     cfgNoise_ = nullptr;
     cfgNoiseValid_ = false;
     sorHostStatus_ = nullptr;
@@ -1825,10 +1826,15 @@ bool Scene::ensureConfigBuffers(std::string& err) {
     cfgLy_ = (ny + 1) / 2;
     cfgLz_ = (nz + 1) / 2;
     const size_t lightCells = static_cast<size_t>(cfgLx_) * cfgLy_ * cfgLz_;
-    return alloc(reinterpret_cast<void**>(&cfgVort_), cells_ * sizeof(float4), "cudaMalloc config vorticity", err) &&
-           alloc(reinterpret_cast<void**>(&cfgLight_), lightCells * sizeof(float), "cudaMalloc config transmittance", err) &&
-           check("clear config vorticity", cudaMemsetAsync(cfgVort_, 0, cells_ * sizeof(float4), stream), err) &&
-           check("clear config transmittance", cudaMemsetAsync(cfgLight_, 0, lightCells * sizeof(float), stream), err);
+    const size_t lightBytes = (lightCells * sizeof(float) + 255) / 256 * 256;
+    const size_t bytes = lightBytes + cfgOccupancyBytes(nx, ny, nz);
+    if (!alloc(reinterpret_cast<void**>(&cfgVort_), cells_ * sizeof(float4), "cudaMalloc config vorticity", err) ||
+        !alloc(reinterpret_cast<void**>(&cfgLight_), bytes, "cudaMalloc config transmittance", err)) {
+        return false;
+    }
+    cfgOcc_ = reinterpret_cast<CfgOccupancy*>(reinterpret_cast<unsigned char*>(cfgLight_) + lightBytes);
+    return check("clear config vorticity", cudaMemsetAsync(cfgVort_, 0, cells_ * sizeof(float4), stream), err) &&
+           check("clear config transmittance", cudaMemsetAsync(cfgLight_, 0, bytes, stream), err);
 }
 
 // One step of this scene inside a FireBatch: the frame's bookkeeping (clocks,
@@ -1891,6 +1897,7 @@ bool Scene::batchStep(BatchScene& d, const FireSettings& s, bool render, std::st
     b.divergence = divergence_;
     b.delta = mgP_[0];
     b.transmittance = cfgLight_;
+    b.occupancy = cfgOcc_;
     b.hdr = hdr_;
     const HdrSlot& slot = slots_[activeSlot_];
     b.slot = slot.ptr;
@@ -1900,6 +1907,7 @@ bool Scene::batchStep(BatchScene& d, const FireSettings& s, bool render, std::st
     b.count[kBatchFaces] = (nx + 1) * (ny + 1) * (nz + 1);
     b.count[kBatchLight] = render ? cfgLx_ * cfgLy_ * cfgLz_ : 0;
     b.count[kBatchPixels] = render ? frameW * frameH : 0;
+    b.count[kBatchBricks] = render ? 32 * cfgOccupancyUnits(nx, ny, nz) : 0;
     d = b;
     cur_ = 1 - cur_;
     vcur_ = 1 - vcur_;
@@ -1920,6 +1928,14 @@ bool Scene::prepareBatched(std::string& err) {
     return cfgNoise_ != nullptr || alloc(reinterpret_cast<void**>(&cfgNoise_), cells_ * sizeof(float4), "cudaMalloc config noise field", err);
 }
 
+// Rays up to which a light or camera ray gets kRayLanes lanes instead of one.
+// Four lanes fill the chip and shorten a ray's chain of dependent loads; past a
+// warp or so per scheduler slot their shuffles and idle lanes cost more.  Dense
+// grids, light + render: 24^3 at 64x64 97 -> 44 us, 61x47x83 at 320x180 124 -> 79,
+// 64^3 at 256x256 179 -> 144 (65,536 camera and 32,768 light rays); 128^3 at
+// 512x512 (262,144 of each) 587 -> 638, 256^3 1,601 -> 1,945.
+constexpr long long kLaneRays = 131072;
+
 // The config physics on the frame's stage ids: advect velocity, advect +
 // react + emit, forces (vorticity, cell accelerations, faces with the walls),
 // divergence, SOR, subtract, transmittance, raymarch, camera response,
@@ -1929,6 +1945,10 @@ bool Scene::runConfigStages(int first, int last, const FrameParams& p, std::stri
     if (!ensureConfigBuffers(err)) return false;
     const int bx = rowThreads(nx);
     const dim3 cells = cellGrid(bx, nx, ny, nz);
+    // Built by this call's light stage from the records that its render stage
+    // reads (the stages that write them come earlier); a call that renders
+    // without it, maybe after the caller has set fields, builds its own.
+    bool occupancyBuilt = false;
     for (int s = first; s <= last; ++s) {
         const ConfigParams c = configParams();
         switch (s) {
@@ -1997,11 +2017,25 @@ bool Scene::runConfigStages(int first, int last, const FrameParams& p, std::stri
                 break;
             case kLightBuild: {
                 const int lbx = rowThreads(cfgLx_);
-                cfgTransmittance<<<dim3((cfgLx_ + lbx - 1) / lbx, cfgLy_, cfgLz_), lbx, 0, stream>>>(cfgLight_, sa_[cur_], c); ++launches_;
+                cfgOccupancyBuild<<<(cfgOccupancyUnits(nx, ny, nz) + 3) / 4, 128, 0, stream>>>(cfgOcc_, sa_[cur_], nullptr, c); ++launches_;
+                occupancyBuilt = true;
+                const long long rays = static_cast<long long>(cfgLx_) * cfgLy_ * cfgLz_;
+                if (rays <= kLaneRays) {
+                    cfgTransmittanceLanes<<<static_cast<int>((rays * kRayLanes + 127) / 128), 128, 0, stream>>>(cfgLight_, sa_[cur_], cfgOcc_, c); ++launches_;
+                } else {
+                    cfgTransmittance<<<dim3((cfgLx_ + lbx - 1) / lbx, cfgLy_, cfgLz_), lbx, 0, stream>>>(cfgLight_, sa_[cur_], cfgOcc_, c); ++launches_;
+                }
                 break;
             }
             case kRender:
-                cfgRaymarch<<<dim3((frameW + 15) / 16, (frameH + 7) / 8), dim3(16, 8), 0, stream>>>(hdr_, sa_[cur_], cfgLight_, c); ++launches_;
+                if (!occupancyBuilt) {
+                    cfgOccupancyBuild<<<(cfgOccupancyUnits(nx, ny, nz) + 3) / 4, 128, 0, stream>>>(cfgOcc_, sa_[cur_], cfgLight_, c); ++launches_;
+                }
+                if (static_cast<long long>(frameW) * frameH <= kLaneRays) {
+                    cfgRaymarchLanes<<<dim3((frameW + 15) / 16, (frameH + 1) / 2), 128, 0, stream>>>(hdr_, sa_[cur_], cfgLight_, cfgOcc_, c); ++launches_;
+                } else {
+                    cfgRaymarch<<<dim3((frameW + 15) / 16, (frameH + 7) / 8), dim3(16, 8), 0, stream>>>(hdr_, sa_[cur_], cfgLight_, cfgOcc_, c); ++launches_;
+                }
                 break;
             case kTonemap:
                 tonemapOverlay<<<dim3((frameW + 15) / 16, (frameH + 15) / 16), dim3(16, 16), 0, stream>>>(bgra_, hdr_, p, 1, 0); ++launches_;
