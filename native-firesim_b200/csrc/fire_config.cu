@@ -709,8 +709,11 @@ __device__ __forceinline__ void cfgRaymarchAt(float4* __restrict__ hdr, const Re
         termR = termG = termB = 0.0f;
         through = 1.0f;
         if (own) evaluate(s);
+        // The ray's own samples only: 0 times an infinite view would be NaN.
 #pragma unroll
-        for (int j = 0; j < LANES; ++j) add(j);
+        for (int j = 0; j < LANES; ++j) {
+            if (LANES == 1 || s0 + j < p.primarySamples) add(j);
+        }
     }
     if (!live || sub != 0) return;
     if (hit && last < p.primarySamples) {  // the samples after the last one add 0 times the view

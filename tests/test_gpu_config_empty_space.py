@@ -70,3 +70,30 @@ def test_passing_over_empty_bricks_changes_no_bit(pkg, abi, dims, frame, kind):
     sim.close()
     for x, y in zip(a, b):
         assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["nothing", "corners", "sparse", "signed", "full", "overflow", "exit"])
+@pytest.mark.parametrize("samples", [1, 10, 96])
+def test_rays_of_four_lanes_equal_rays_of_one(pkg, abi, samples, kind):
+    """A frame of 648 x 360 has more rays than get four lanes each; the middle
+    pixels of its 9 x 9 blocks are the rays of the 72 x 40 frame.  exit: matter
+    at the box's far wall only, where the view turns infinite at the last sample."""
+    dims = (40, 33, 37)
+    fields = _state(dims, "nothing" if kind == "exit" else kind, np.random.default_rng(5))
+    if kind == "exit":
+        fields["soot"][0] = fields["soot"][-1] = fields["soot"][:, :, 0] = fields["soot"][:, :, -1] = -3.0e4
+    hdr = []
+    for frame in ((72, 40), (648, 360)):
+        sim = pkg.FireSim(*frame, *dims)
+        p = abi.default_physics(*dims)
+        p.mode, p.primarySamples = 1, samples
+        sim.set_physics(p)
+        sim.reset()
+        for n, a in fields.items():
+            sim.set(n, a)
+        sim.stages("light_build", "render", abi.FireSettings(width=frame[0], height=frame[1]), 0.0)
+        hdr.append(sim.get("hdr").reshape(frame[1], frame[0], 4))
+        sim.close()
+    few, many = hdr[0], np.ascontiguousarray(hdr[1][4::9, 4::9])
+    assert np.array_equal(np.isnan(few), np.isnan(many))
+    assert np.array_equal(np.where(np.isnan(few), 0.0, few), np.where(np.isnan(many), 0.0, many))
