@@ -323,6 +323,7 @@ struct MgPlan {
     int gridLevels;  // max over the scenes of tail
     int maxCycles, pre, post, gated;
     float tolerance;
+    int l2Cells;             // a level of more cells exceeds the L2 (p, its other buffer and the rhs): tiles are prefetched
     int tile[kMgMaxLevels];  // index of the level's tile shape in kMgTiles
     int tileUnits[kMgMaxLevels][kMgMaxScenes + 1];
     int fineUnits[kMgMaxLevels][kMgMaxScenes + 1];

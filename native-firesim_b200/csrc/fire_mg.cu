@@ -648,11 +648,13 @@ struct TileJob {
     float* dst;
     const float* correction;
     float *coarseRhs, *coarseP;
-    int unit, red, x0, y0, z0;
+    int unit, red, prefetch, x0, y0, z0;
 };
 // The CTA's tile and the next one, in shared memory: operands that the stages
-// below read from there cost no registers, and a thread without cells prepares
-// the next tile while the others smooth (0.9 us of latency a tile else).
+// below read from there cost no registers, and the last thread prepares the next
+// tile while the others load (0.9 us of latency a tile else).  A block barrier
+// lies between every write and the reads of it, and between those and the next
+// write.
 __shared__ TileJob sTile[2];
 
 // The residuals of the cells x (even) and x + 1 of row (y, z), both in slot k.
@@ -870,30 +872,29 @@ __device__ __noinline__ void tileCorrect() {
     __syncthreads();
 }
 
-// The next tile's rows into L2, by the warps that have no columns, where the
-// level's p, its other buffer and its rhs exceed the L2: a V-cycle at 256^3
-// (201 MB) went 666 -> 647 us.  At 192^3 (85 MB), where the rows are in L2, it
-// went 317 -> 320 us, at 128^3 148 -> 151.
-constexpr int kMgL2Cells = (126 << 20) / 12;
+// The next tile's rows into L2, by the warps from the first without a column on,
+// or the last one.  Its operands were written before the barrier that ends the
+// load of the tile in hand.
 template <int TX, int TY, int TZ>
 __device__ __forceinline__ void tilePrefetch(int buf, int total) {
     using S = TileShape<TX, TY, TZ>;
     constexpr int kFirst = S::GROUPS * S::COLS / 32 * 32 < kMgThreads - 32 ? S::GROUPS * S::COLS / 32 * 32 : kMgThreads - 32;
     if (threadIdx.x < kFirst) return;
-    __syncwarp();
     const TileJob& job = sTile[buf];
     if (job.unit >= total) return;
     const int nx = job.L.nx, ny = job.L.ny, nz = job.L.nz;
-    const int x = max(job.x0 - S::H, 0);
+    const int x = max(job.x0 - S::H, 0), end = min(job.x0 + TX + S::H, nx);
     for (int i = threadIdx.x - kFirst; i < S::RY * S::RZ; i += kMgThreads - kFirst) {
         const int lz = i / S::RY, y = job.y0 - S::H + i - lz * S::RY, z = job.z0 - S::H + lz;
         if (y < 0 || y >= ny || z < 0 || z >= nz) continue;
         const int g = (z * ny + y) * nx;
-        const int last = min(job.x0 + TX + S::H, nx) - 1;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + x));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + x));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + last));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + last));
+        // Every 128-byte line of the row: from its first cell by 32, and its last cell.
+        for (int at = x; at < end; at += 32) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + at));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + at));
+        }
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + end - 1));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + end - 1));
     }
 }
 
@@ -909,7 +910,7 @@ __device__ __noinline__ void tileSmooth(int buf, int first, int count, int total
     // With the restriction the cells beside the tile stay valid to the end.
     const int beyond = job.coarseRhs != nullptr ? 1 : 0;
     if (job.correction != nullptr) tileCorrect<TX, TY, TZ>();
-    if (L.nx * L.ny * L.nz > kMgL2Cells) tilePrefetch<TX, TY, TZ>(buf ^ 1, total);
+    if (job.prefetch != 0) tilePrefetch<TX, TY, TZ>(buf ^ 1, total);
     for (int s = 0; s < count; ++s) {
         tileHalfSweep<TX, TY, TZ>(L, smem, x0, y0, z0, (first + s) & 1, count - 1 - s + beyond);
         __syncthreads();
@@ -1016,6 +1017,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             job.coarseRhs = restrict ? S.rhs[l + 1] : nullptr;
             job.coarseP = S.p[l + 1];
             job.red = redFirst && l + 1 < S.tail ? 1 : 0;
+            job.prefetch = L.nx * L.ny * L.nz > plan->l2Cells ? 1 : 0;
             const int tx = shape == 0 ? kMgTiles[0].x : shape == 1 ? kMgTiles[1].x : shape == 2 ? kMgTiles[2].x : kMgTiles[3].x;
             const int ty = shape == 0 ? kMgTiles[0].y : shape == 1 ? kMgTiles[1].y : shape == 2 ? kMgTiles[2].y : kMgTiles[3].y;
             const int tz = shape == 0 ? kMgTiles[0].z : shape == 1 ? kMgTiles[1].z : shape == 2 ? kMgTiles[2].z : kMgTiles[3].z;
@@ -1030,6 +1032,9 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
         if (threadIdx.x == kPreparer) prepare(0, blockIdx.x);
         __syncthreads();
         for (int buf = 0; sTile[buf].unit < total; buf ^= 1) {
+            // Before the load: the barrier that ends it publishes the next tile's
+            // operands, and the one that ended the last tile freed their place.
+            if (threadIdx.x == kPreparer) prepare(buf ^ 1, sTile[buf].unit + gridDim.x);
             if (shape == 0) {
                 tileLoad<32, 16, 16>(buf);
             } else if (shape == 1) {
@@ -1039,7 +1044,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             } else {
                 tileLoad<8, 8, 4>(buf);
             }
-            if (threadIdx.x == kPreparer) prepare(buf ^ 1, sTile[buf].unit + gridDim.x);
             if (shape == 0) {
                 tileSmooth<32, 16, 16>(buf, first, count, total);
             } else if (shape == 1) {

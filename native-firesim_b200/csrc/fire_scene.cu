@@ -761,14 +761,16 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
     }
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess && dScenes_ == nullptr) {
-        int sms = 0, coop = 0;
+        int sms = 0, coop = 0, l2 = 0;
         e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
         if (e == cudaSuccess && !coop) {
             err = "multigrid: the device cannot run the persistent solve (no cooperative launch)";
             return false;
         }
         sms_ = sms;
+        l2Cells_ = l2 / static_cast<int>(3 * sizeof(float));
         if (e == cudaSuccess) {
             e = cudaFuncSetAttribute(mgSolve, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMgTailSmemMax));
         }
@@ -804,6 +806,7 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
     plan.pre = pre;
     plan.post = post;
     plan.gated = tolerance > 0.0 ? 1 : 0;
+    plan.l2Cells = l2Cells_;
     plan.tolerance = static_cast<float>(tolerance);
     size_t smem = 0;
     for (int s = 0; s < n; ++s) {

@@ -73,7 +73,7 @@ private:
     int slot_ = 0;
     bool planned_ = false;
     size_t smem_ = 0;
-    int grid_ = 0, sms_ = 0;
+    int grid_ = 0, sms_ = 0, l2Cells_ = 0;
     unsigned long long waitNs_ = 1000000000ull;
 };
 
