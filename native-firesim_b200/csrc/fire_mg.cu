@@ -652,9 +652,9 @@ struct TileJob {
 };
 // The CTA's tile and the next one, in shared memory: operands that the stages
 // below read from there cost no registers, and the last thread prepares the next
-// tile while the others load (0.9 us of latency a tile else).  A block barrier
-// lies between every write and the reads of it, and between those and the next
-// write.
+// tile while the others smooth (0.9 us of latency a tile else; before the load it
+// delayed that, a V-cycle at 128^3 157 us instead of 146).  A block barrier lies
+// between every write and the reads of it, and between those and the next write.
 __shared__ TileJob sTile[2];
 
 // The residuals of the cells x (even) and x + 1 of row (y, z), both in slot k.
@@ -872,9 +872,14 @@ __device__ __noinline__ void tileCorrect() {
     __syncthreads();
 }
 
-// The next tile's rows into L2, by the warps from the first without a column on,
-// or the last one.  Its operands were written before the barrier that ends the
-// load of the tile in hand.
+// The next tile's rows into L2 (the lines of a row's first and last cell; its
+// other lines come with the neighbouring tiles), by the warps that have no
+// columns, or the last one, where the level's p, its other buffer and its rhs
+// exceed the L2.  After the first half sweep, whose barrier orders the next tile's
+// operands before these reads.  A V-cycle at 256^3 (201 MB) takes 636 us with it
+// and 660 without, at 240x232x224 (150 MB) 591 and 602, at 320^3 1221 and 1284
+// (every line of the rows, by one warp: 685, 635 and 1366).  At 192^3 (85 MB), where the
+// rows are in L2, it went 317 -> 320 us, at 128^3 148 -> 151.
 template <int TX, int TY, int TZ>
 __device__ __forceinline__ void tilePrefetch(int buf, int total) {
     using S = TileShape<TX, TY, TZ>;
@@ -883,18 +888,15 @@ __device__ __forceinline__ void tilePrefetch(int buf, int total) {
     const TileJob& job = sTile[buf];
     if (job.unit >= total) return;
     const int nx = job.L.nx, ny = job.L.ny, nz = job.L.nz;
-    const int x = max(job.x0 - S::H, 0), end = min(job.x0 + TX + S::H, nx);
+    const int x = max(job.x0 - S::H, 0), last = min(job.x0 + TX + S::H, nx) - 1;
     for (int i = threadIdx.x - kFirst; i < S::RY * S::RZ; i += kMgThreads - kFirst) {
         const int lz = i / S::RY, y = job.y0 - S::H + i - lz * S::RY, z = job.z0 - S::H + lz;
         if (y < 0 || y >= ny || z < 0 || z >= nz) continue;
         const int g = (z * ny + y) * nx;
-        // Every 128-byte line of the row: from its first cell by 32, and its last cell.
-        for (int at = x; at < end; at += 32) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + at));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + at));
-        }
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + end - 1));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + end - 1));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + x));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + x));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.src + g + last));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(job.rhs + g + last));
     }
 }
 
@@ -910,10 +912,10 @@ __device__ __noinline__ void tileSmooth(int buf, int first, int count, int total
     // With the restriction the cells beside the tile stay valid to the end.
     const int beyond = job.coarseRhs != nullptr ? 1 : 0;
     if (job.correction != nullptr) tileCorrect<TX, TY, TZ>();
-    if (job.prefetch != 0) tilePrefetch<TX, TY, TZ>(buf ^ 1, total);
     for (int s = 0; s < count; ++s) {
         tileHalfSweep<TX, TY, TZ>(L, smem, x0, y0, z0, (first + s) & 1, count - 1 - s + beyond);
         __syncthreads();
+        if (s == 0 && job.prefetch != 0) tilePrefetch<TX, TY, TZ>(buf ^ 1, total);
     }
     if (beyond != 0) tileRestrict<TX, TY, TZ>(buf);
     const bool whole = (L.nx & 3) == 0;
@@ -1032,9 +1034,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
         if (threadIdx.x == kPreparer) prepare(0, blockIdx.x);
         __syncthreads();
         for (int buf = 0; sTile[buf].unit < total; buf ^= 1) {
-            // Before the load: the barrier that ends it publishes the next tile's
-            // operands, and the one that ended the last tile freed their place.
-            if (threadIdx.x == kPreparer) prepare(buf ^ 1, sTile[buf].unit + gridDim.x);
             if (shape == 0) {
                 tileLoad<32, 16, 16>(buf);
             } else if (shape == 1) {
@@ -1044,6 +1043,9 @@ __global__ void __launch_bounds__(kMgThreads, 1) mgSolve(const MgScene* __restri
             } else {
                 tileLoad<8, 8, 4>(buf);
             }
+            // The barrier that ended the last tile freed the place; those of the
+            // half sweeps publish it.
+            if (threadIdx.x == kPreparer) prepare(buf ^ 1, sTile[buf].unit + gridDim.x);
             if (shape == 0) {
                 tileSmooth<32, 16, 16>(buf, first, count, total);
             } else if (shape == 1) {
