@@ -809,8 +809,10 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
     plan.l2Cells = l2Cells_;
     plan.tolerance = static_cast<float>(tolerance);
     size_t smem = 0;
+    bool globalTail = false;  // some scene's tail runs in its global buffers
     for (int s = 0; s < n; ++s) {
         const MgScene& S = scenes[s];
+        globalTail = globalTail || S.tailMode == kMgTailGlobal;
         plan.gridLevels = std::max(plan.gridLevels, S.tail);
         size_t tailFloats = 0;
         for (int l = S.tail; l < S.levels; ++l) tailFloats += 2 * static_cast<size_t>(S.lv[l].nx) * S.lv[l].ny * S.lv[l].nz;
@@ -830,9 +832,13 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
     // plus a time per cell of the region (measured: 9.3 us for 32x16x16's 23,040).
     // Large tiles waste the least on halos; where they would leave SMs idle or
     // end in a nearly empty wave, smaller ones finish sooner (32^3: 8x8x4 3.6 us).
+    // Beside a tail in global buffers the largest is left out: its shared memory
+    // (197 KB of the SM's 256 with the L1) leaves that tail, nearly all of such a
+    // cycle, hardly any L1 (250x198x154 34.7 ms a cycle with it, 22.9 without;
+    // 99x100x102 4.7 and 3.5 ms; the smaller shapes alone 22.9 and 3.5).
     for (int l = 0; l < plan.gridLevels; ++l) {
         double best = 0.0;
-        for (int k = 0; k < kMgTileShapes; ++k) {
+        for (int k = globalTail ? 1 : 0; k < kMgTileShapes; ++k) {
             long long tiles = 0;
             for (int s = 0; s < n; ++s) {
                 if (l < scenes[s].tail) tiles += mgTiles(kMgTiles[k], scenes[s].lv[l]);
