@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -1009,14 +1010,22 @@ bool Scene::runMetrics(const FrameParams& p, std::string& err) {
 
 namespace {
 
+// Lattice coordinates up to which tables are built (reached about 2e8 s after the
+// start).  Past INT_MAX a table's origin is undefined, and the kernels' saturating
+// conversion of a coordinate could land inside the table of another.
+constexpr double kLatticeReach = 1.0e9;
+bool withinReach(double x) { return std::fabs(x) <= kLatticeReach; }
+
 // Lattice of one 2D fbm call site whose octave-0 inputs lie in
 // [pxLo, pxHi] x [pyLo, pyHi]; later octaves map the range through the octave
 // step (x * 2.03 + 17.7, y * 2.01 - 9.2, src/fire_cuda.cu:423-432), widened by
 // one lattice cell per octave for rounding.  Entries past the edges are
-// hashed in place by fbmLattice, so the margins only affect speed.
+// hashed in place by fbmLattice, so the margins only affect speed.  INT_MAX where
+// an end is beyond kLatticeReach or not a number: no table fits there.
 int planLattice(double pxLo, double pxHi, double pyLo, double pyHi, HashLattice2& L) {
     int offset = 0;
     for (int o = 0; o < kFbmOctaves; ++o) {
+        if (!withinReach(pxLo) || !withinReach(pxHi) || !withinReach(pyLo) || !withinReach(pyHi)) return INT_MAX;
         L.ox[o] = static_cast<int>(std::floor(pxLo)) - 2;
         L.oy[o] = static_cast<int>(std::floor(pyLo)) - 2;
         L.sx[o] = static_cast<int>(std::floor(pxHi)) - L.ox[o] + 4;
@@ -1066,7 +1075,8 @@ bool Scene::sourceLattice(const FrameParams& p, HashLattice2& l) const {
 // The tables of the raymarch's noise fields for this frame: per field and
 // octave every lattice cell that a sample position in [0, 1]^3 can reach, one
 // cell wider on each side (a cell outside is hashed in place, so the margin
-// affects speed only).  The sizes do not depend on the time (1.46 M entries).
+// affects speed only; an octave beyond kLatticeReach has no table).  The room
+// does not depend on the time (1.46 M entries).
 // They lie in the force scratch, which no stage of a frame uses, where the grid
 // has that many cells; else in a buffer that the first frame allocates, and a
 // frame goes without where that fails or the stream is being captured.
@@ -1082,19 +1092,21 @@ bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
                              {-t * 0.72, -t * 1.08, t * 0.32}};
     const double span[4][3] = {{7.0, 5.0, 9.0}, {8.0, 8.0, 6.0}, {42.0, 54.0, 43.0}, {15.0, 13.0, 17.0}};
     const double scale[3] = {2.03, 2.01, 2.07}, shift[3] = {17.7, -9.2, 5.1};
-    int total = 0;
+    int total = 0, capacity = 0;
     for (int f = 0; f < 4; ++f) {
         double a[3] = {lo[f][0], lo[f][1], lo[f][2]}, w[3] = {span[f][0], span[f][1], span[f][2]};
         for (int o = 0; o < kRenderOctaves; ++o) {
             const int k = f * kRenderOctaves + o;
             int org[3], size[3];
+            bool within = true;
             for (int d = 0; d < 3; ++d) {
-                org[d] = static_cast<int>(std::floor(a[d])) - 1;
+                within = within && withinReach(a[d]);
+                org[d] = within ? static_cast<int>(std::floor(a[d])) - 1 : 0;
                 size[d] = static_cast<int>(std::ceil(w[d])) + 3 + (d == 2 ? 1 : 0);
                 a[d] = a[d] * scale[d] + shift[d];
                 w[d] *= scale[d];
             }
-            const bool table = f != 2 || o + 1 < kRenderOctaves;
+            const bool room = f != 2 || o + 1 < kRenderOctaves, table = room && within;
             n.ox[k] = org[0];
             n.oy[k] = org[1];
             n.oz[k] = org[2];
@@ -1103,9 +1115,10 @@ bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
             n.sz[k] = table ? size[2] : 0;
             n.offset[k] = total;
             total += n.sx[k] * n.sy[k] * n.sz[k];
+            capacity += room ? size[0] * size[1] * size[2] : 0;
         }
     }
-    if (cells_ >= static_cast<size_t>(total)) {
+    if (cells_ >= static_cast<size_t>(capacity)) {
         n.values = contrib_;
         n.total = total;
         return true;
@@ -1117,7 +1130,7 @@ bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
             return false;
         }
         std::string ignored;
-        if (!alloc(reinterpret_cast<void**>(&renderNoise_), static_cast<size_t>(total) * sizeof(float4), "cudaMalloc render noise", ignored)) {
+        if (!alloc(reinterpret_cast<void**>(&renderNoise_), static_cast<size_t>(capacity) * sizeof(float4), "cudaMalloc render noise", ignored)) {
             cudaGetLastError();
             renderNoiseRefused_ = true;
             return false;
