@@ -228,12 +228,15 @@ __device__ __forceinline__ void tailSmoothLanes(float* __restrict__ p, const flo
 // goes to tailSmoothLanes; one of at most 128 cells is relaxed by the first
 // warp alone, with warp barriers; otherwise by the whole CTA.  skipFirst:
 // the first colour-0 half sweep was already done (from p = 0, by whoever
-// wrote the level's rhs).  The loops are not unrolled: each level's smoothing is
-// code of its own, and by four its fetches cost more than the loads in flight
-// gave (a V-cycle 150 -> 147 us at 128^3, 155 -> 141 us at 200x24x216).
+// wrote the level's rhs).  In shared memory the loops are not unrolled: each
+// level's smoothing is code of its own, and by four its fetches cost more than
+// the loads in flight gave (a V-cycle 150 -> 147 us at 128^3, 155 -> 141 us at
+// 200x24x216).  In global memory the loads in flight count (a V-cycle at
+// 150x140x61 4.20 ms without, 4.16 ms by four).
 template <bool PG, bool RG>
 __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* __restrict__ rhs, const MgLevel L, int sweeps,
                                            bool skipFirst) {
+    constexpr int kUnroll = PG ? 4 : 1;
     const int cols = L.nx * L.ny;
     if (!PG && cols * L.nz <= 32) {
         tailSmoothLanes<RG>(p, rhs, L, sweeps, skipFirst);
@@ -258,7 +261,7 @@ __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* _
             for (int s = 0; s < sweeps; ++s) {
                 for (int colour = skipFirst && s == 0 ? 1 : 0; colour < 2; ++colour) {
                     if (m.active) {
-#pragma unroll 1
+#pragma unroll kUnroll
                         for (int z = z0 ^ colour; z < L.nz; z += dz) {
                             const int i = m.col + z * cols;
                             p[i] = weightedSum(load, tailLoad<RG>(rhs, i), L, i, x, y, z, load(i)) * L.invDiag;
@@ -272,7 +275,7 @@ __device__ __forceinline__ void tailSmooth(float* __restrict__ p, const float* _
                 for (int colour = skipFirst && s == 0 ? 1 : 0; colour < 2; ++colour) {
                     for (int col = m.col; col < cols; col += m.colStride) {
                         const int y = col / L.nx, x = col - y * L.nx;
-#pragma unroll 1
+#pragma unroll kUnroll
                         for (int z = (colour + x + y) & 1; z < L.nz; z += 2) {
                             const int i = col + z * cols;
                             p[i] = weightedSum(load, tailLoad<RG>(rhs, i), L, i, x, y, z, load(i)) * L.invDiag;
