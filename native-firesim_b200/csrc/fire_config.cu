@@ -415,72 +415,98 @@ __global__ void __launch_bounds__(128) cfgApplyForces(FaceT* __restrict__ uOut, 
 // brick.  The exceptions: a step, a light colour or a transmittance so large that
 // 0 times it could be NaN evaluates every sample, and so does a pixel whose
 // remaining view is infinite or NaN, from there on.  Where half of the bricks are
-// set, only the cut to the box is made.  Measured (light, render): 128^3 after 60
-// steps 141 -> 44 and 434 -> 110 us, 256^3 half 442 -> 89 and 397 -> 91 us; of it
-// the build 9 us at 64^3, 13 at 128^3, 80 at 256^3 (floor 41: the record once).
-// With every brick set 554 -> 568 us in sum at 128^3.
+// set, only the cut to the box is made, and a grid that is largely full (48 of 64
+// cells spread over it) takes every sample: its records are not read, and the
+// kernels run the plain loop, whose samples overlap better than the cut one's
+// (full 192^3, 65,536 rays of one lane: 213 us in the cut loop, 136 in the plain
+// one).  Measured (light, render, each with its build): 128^3 after 40 steps 138 ->
+// 31 and 440 -> 95 us, 256^3 1014 -> 86 and 486 -> 138 us; full grids, in sum, 128^3
+// 561 and 557 us, 256^3 1493 and 1500, 64^3 159 and 131.  The build takes 4 us on a
+// full grid, 10 at 128^3 and 65 at 256^3 otherwise (floor 41: the record once).
 
 __device__ __forceinline__ bool seen(float4 r) { return (r.x != 0.0f) | (r.y != 0.0f) | (r.w != 0.0f); }
 
-// One warp's unit of the build (cfgOccupancyUnits); tr: also checks that every
-// transmittance is regular.  Bound by its reads of record a, (5/4)^2 of them
-// through L2.  The last warp to finish publishes the box and clears the
-// accumulators for the next build.
+// One warp's share of the build: the units (cfgOccupancyUnits) warp, warp + warps,
+// ...; tr: also checks that every transmittance is regular.  Bound by its reads
+// of record a, (5/4)^2 of them through L2: a warp keeps the box and the count of
+// its units in registers, as the atomics of every unit took as long as the reads.
+// The last warp to finish publishes the box and clears the accumulators for the
+// next build.
 __device__ __forceinline__ void cfgOccupancyAt(CfgOccupancy* occ, const Rec4* __restrict__ a, const float* __restrict__ tr,
-                                               const ConfigParams& p, int unit, int lane) {
+                                               const ConfigParams& p, int warp, int warps, int lane) {
     const int bx = cfgBricks(p.nx), by = cfgBricks(p.ny), bz = cfgBricks(p.nz);
     const int perRow = (bx + 6) / 7;
     const int units = perRow * by * bz;
-    const int row = unit / perRow, chunk = unit - row * perRow;
-    const int Z = row / by, Y = row - Z * by;
-    const int x = min(28 * chunk + lane, p.nx - 1);
-    // Past the grid's ends the last cell again; all 25 loads in flight.
-    bool any = false;  // (|, not ||: a short circuit would wait for each load)
+    // Every warp looks at the same cells of the same records, so all take the same way.
+    int full = 0;
 #pragma unroll
-    for (int dz = 0; dz < 5; ++dz) {
+    for (int k = 0; k < 2; ++k) {
+        const int x = (2 * (lane & 3) + 1) * p.nx / 8, y = (2 * ((lane >> 2) & 3) + 1) * p.ny / 8, z = (2 * (2 * k + (lane >> 4)) + 1) * p.nz / 8;
+        full += __popc(__ballot_sync(0xffffffffu, seen(ldv(a + faceIndex(x, y, z, p.nx, p.ny)))));
+    }
+    if (full >= 48) {
+        if (warp == 0 && lane == 0) occ->look = kCfgEvery;
+        return;
+    }
+    unsigned lo = 0u, hi = 0u, count = 0u;  // the set bricks' ends in the axis lane % 3, and their number
+    for (int unit = warp; unit < units; unit += warps) {
+        const int row = unit / perRow, chunk = unit - row * perRow;
+        const int Z = row / by, Y = row - Z * by;
+        const int x = min(28 * chunk + lane, p.nx - 1);
+        // Past the grid's ends the last cell again; all 25 loads in flight.
+        bool any = false;  // (|, not ||: a short circuit would wait for each load)
 #pragma unroll
-        for (int dy = 0; dy < 5; ++dy) any |= seen(ldv(a + faceIndex(x, min(4 * Y + dy, p.ny - 1), min(4 * Z + dz, p.nz - 1), p.nx, p.ny)));
+        for (int dz = 0; dz < 5; ++dz) {
+#pragma unroll
+            for (int dy = 0; dy < 5; ++dy) any |= seen(ldv(a + faceIndex(x, min(4 * Y + dy, p.ny - 1), min(4 * Z + dz, p.nz - 1), p.nx, p.ny)));
+        }
+        const unsigned cells = __ballot_sync(0xffffffffu, any);
+        const int X = 7 * chunk + lane;
+        bool set = false;
+        if (lane < 7 && X < bx) {
+            set = ((cells >> (4 * lane)) & 31u) != 0u;
+            reinterpret_cast<unsigned char*>(occ + 1)[(Z * by + Y) * bx + X] = set ? 1 : 0;
+        }
+        const unsigned f = __ballot_sync(0xffffffffu, set);
+        if (f == 0u) continue;
+        count += static_cast<unsigned>(__popc(f));
+        const int axis = lane % 3;
+        const int first = axis == 0 ? 7 * chunk + __ffs(static_cast<int>(f)) - 1 : axis == 1 ? Y : Z;
+        const int last = axis == 0 ? 7 * chunk + 31 - __clz(static_cast<int>(f)) : axis == 1 ? Y : Z;
+        lo = max(lo, (1u << 20) - static_cast<unsigned>(first));
+        hi = max(hi, static_cast<unsigned>(last) + 1u);
     }
-    const unsigned cells = __ballot_sync(0xffffffffu, any);
-    const int X = 7 * chunk + lane;
-    bool set = false;
-    if (lane < 7 && X < bx) {
-        set = ((cells >> (4 * lane)) & 31u) != 0u;
-        reinterpret_cast<unsigned char*>(occ + 1)[(Z * by + Y) * bx + X] = set ? 1 : 0;
-    }
-    const unsigned f = __ballot_sync(0xffffffffu, set);
     bool irregular = false;
     if (tr != nullptr) {
-        const int count = p.lx * p.ly * p.lz;
-        for (int i = unit * 32 + lane; i < count; i += units * 32) irregular = irregular || !(fabsf(__ldg(tr + i)) <= 1e30f);
+        const int n = p.lx * p.ly * p.lz;
+        for (int i = warp * 32 + lane; i < n; i += min(warps, units) * 32) irregular = irregular || !(fabsf(__ldg(tr + i)) <= 1e30f);
     }
     irregular = __any_sync(0xffffffffu, irregular);
     // Lanes 0-2 the box's low ends, 3-5 its high ends.
-    if (lane == 7 && f != 0u) atomicAdd(&occ->accSet, static_cast<unsigned>(__popc(f)));
-    if (f != 0u && lane < 6) {
-        const int axis = lane % 3;
-        const int lo = axis == 0 ? 7 * chunk + __ffs(static_cast<int>(f)) - 1 : axis == 1 ? Y : Z;
-        const int hi = axis == 0 ? 7 * chunk + 31 - __clz(static_cast<int>(f)) : axis == 1 ? Y : Z;
-        atomicMax(&occ->acc[lane], lane < 3 ? (1u << 20) - static_cast<unsigned>(lo) : static_cast<unsigned>(hi) + 1u);
-    }
+    if (lane == 7 && count != 0u) atomicAdd(&occ->accSet, count);
+    if (lane < 6 && count != 0u) atomicMax(&occ->acc[lane], lane < 3 ? lo : hi);
     if (irregular && lane == 6) atomicOr(&occ->accIrregular, 1u);
     __threadfence();
     __syncwarp();
+    const unsigned participants = static_cast<unsigned>(min(warps, units));
     unsigned done = 0u;
-    if (lane == 0) done = atomicInc(&occ->done, static_cast<unsigned>(units) - 1u);  // wraps to 0 for the next build
-    if (__shfl_sync(0xffffffffu, done, 0) != static_cast<unsigned>(units) - 1u) return;
+    if (lane == 0) done = atomicInc(&occ->done, participants - 1u);  // wraps to 0 for the next build
+    if (__shfl_sync(0xffffffffu, done, 0) != participants - 1u) return;
     __threadfence();
     if (lane < 6) occ->box[lane] = atomicExch(&occ->acc[lane], 0u);
     if (lane == 6) occ->irregular = atomicExch(&occ->accIrregular, 0u);
     // Set bricks in half the grid or more: asking for each sample costs more than it saves.
-    if (lane == 7) occ->dense = atomicExch(&occ->accSet, 0u) >= static_cast<unsigned>(bx) * static_cast<unsigned>(by) * static_cast<unsigned>(bz) / 2u ? 1u : 0u;
+    if (lane == 7) {
+        const unsigned bricks = static_cast<unsigned>(bx) * static_cast<unsigned>(by) * static_cast<unsigned>(bz);
+        occ->look = atomicExch(&occ->accSet, 0u) >= bricks / 2u ? kCfgBox : kCfgAsk;
+    }
 }
 
 __global__ void __launch_bounds__(128) cfgOccupancyBuild(CfgOccupancy* occ, const Rec4* __restrict__ a, const float* __restrict__ tr,
                                                          ConfigParams p) {
-    const int unit = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (unit >= cfgOccupancyUnits(p.nx, p.ny, p.nz)) return;
-    cfgOccupancyAt(occ, a, tr, p, unit, threadIdx.x & 31);
+    const int warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (warp >= cfgOccupancyUnits(p.nx, p.ny, p.nz)) return;
+    cfgOccupancyAt(occ, a, tr, p, warp, gridDim.x * 4, threadIdx.x & 31);
 }
 
 // The samples first .. last - 1 of a ray (origin + direction * (t0 + (s + 0.5)
@@ -518,7 +544,7 @@ __device__ __forceinline__ void samplesInBox(const CfgOccupancy* occ, const Conf
 }
 
 // Rays are taken by a lane each or, where that leaves the chip short of warps
-// (cfgLanes), by kRayLanes lanes each: a lane evaluates every kRayLanes-th
+// (kLightLaneRays, pixelLanes), by kRayLanes lanes each: a lane evaluates every kRayLanes-th
 // sample, and all of them add the samples' terms in order, passed by shuffles,
 // so the sums are the same to the bit.  sub is the lane's number in its ray; the
 // warp's rays walk their samples together, full warps only.
@@ -554,7 +580,10 @@ __device__ __forceinline__ float fromLane(float v, int j) {
 // Transmittance toward the point light from the centre of each 2x2x2 block of
 // cells: lightSamples midpoint samples of extinction * S + fuelExtinction * F
 // along the segment, clipped where it leaves the grid box.
-template <int LANES>
+// SKIP: with an occupancy, else every sample.  BESIDE: compiled beside the form
+// with one, where the plain loop of a kernel of its own came out slower (full
+// 128^3 181 us instead of 144).
+template <int LANES, bool SKIP, bool BESIDE = false>
 __device__ __forceinline__ void cfgTransmittanceAt(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ, const ConfigParams& p,
                                                    int lx, int ly, int lz, int sub, bool live) {
     const float px = 2.0f * static_cast<float>(lx) + 1.0f, py = 2.0f * static_cast<float>(ly) + 1.0f, pz = 2.0f * static_cast<float>(lz) + 1.0f;
@@ -572,63 +601,93 @@ __device__ __forceinline__ void cfgTransmittanceAt(float* __restrict__ tr, const
     seg = fmaxf(seg, 0.0f);
     const float ds = seg / static_cast<float>(p.lightSamples);
     float tau = 0.0f;
-    const bool skip = ds < 1e30f, ask = skip && occ->dense == 0u;
-    int first = 0, last = p.lightSamples;
-    if (skip) {
-        const float origin[3] = {px, py, pz}, dir[3] = {rx, ry, rz};
-        samplesInBox(occ, p, origin, dir, 0.0f, ds, p.lightSamples, first, last);
-    }
-    if (!apart || !live) first = last = 0;
-    const int bx = cfgBricks(p.nx), by = cfgBricks(p.ny);
-    int from = last > first ? first : p.lightSamples, to = last;
-    widen<LANES>(from, to);
-    if (LANES == 1 && !ask) {  // no branch in the loop, so that samples overlap
-        for (int s = first; s < last; ++s) {
+    if constexpr (LANES == 1 && !SKIP && !BESIDE) {
+        if (apart) {
+            for (int s = 0; s < p.lightSamples; ++s) {
+                const float at = (static_cast<float>(s) + 0.5f) * ds;
+                const float4 r = recordAt(a, p, px + rx * at, py + ry * at, pz + rz * at);
+                tau = tau + (p.extinction * r.w + p.fuelExtinction * r.y) * ds;
+            }
+        }
+    } else {
+        const unsigned look = SKIP ? occ->look : static_cast<unsigned>(kCfgEvery);
+        const bool skip = look != kCfgEvery && ds < 1e30f, ask = skip && look == kCfgAsk;
+        int first = 0, last = p.lightSamples;
+        if (skip) {
+            const float origin[3] = {px, py, pz}, dir[3] = {rx, ry, rz};
+            samplesInBox(occ, p, origin, dir, 0.0f, ds, p.lightSamples, first, last);
+        }
+        if (!apart || !live) first = last = 0;
+        const int bx = cfgBricks(p.nx), by = cfgBricks(p.ny);
+        int from = last > first ? first : p.lightSamples, to = last;
+        widen<LANES>(from, to);
+        if (LANES == 1 && !ask) {  // no branch in the loop, so that samples overlap
+            for (int s = first; s < last; ++s) {
+                const float at = (static_cast<float>(s) + 0.5f) * ds;
+                const float4 r = recordAt(a, p, px + rx * at, py + ry * at, pz + rz * at);
+                tau = tau + (p.extinction * r.w + p.fuelExtinction * r.y) * ds;
+            }
+            to = from;
+        }
+        for (int s0 = from; s0 < to; s0 += LANES) {
+            const int s = s0 + sub;
             const float at = (static_cast<float>(s) + 0.5f) * ds;
-            const float4 r = recordAt(a, p, px + rx * at, py + ry * at, pz + rz * at);
-            tau = tau + (p.extinction * r.w + p.fuelExtinction * r.y) * ds;
-        }
-        to = from;
-    }
-    for (int s0 = from; s0 < to; s0 += LANES) {
-        const int s = s0 + sub;
-        const float at = (static_cast<float>(s) + 0.5f) * ds;
-        const auto c = recordCorners(p, px + rx * at, py + ry * at, pz + rz * at);
-        bool own = s >= first && s < last;
-        if (own && ask) own = brickSeen(occ, c, bx, by);
-        if (!anyOf<LANES>(own)) continue;
-        float term = 0.0f;
-        if (own) {
-            const float4 r = trilinearRec(a, c, p.nx, p.ny);
-            term = (p.extinction * r.w + p.fuelExtinction * r.y) * ds;
-        }
+            const auto c = recordCorners(p, px + rx * at, py + ry * at, pz + rz * at);
+            bool own = s >= first && s < last;
+            if (own && ask) own = brickSeen(occ, c, bx, by);
+            if (!anyOf<LANES>(own)) continue;
+            float term = 0.0f;
+            if (own) {
+                const float4 r = trilinearRec(a, c, p.nx, p.ny);
+                term = (p.extinction * r.w + p.fuelExtinction * r.y) * ds;
+            }
 #pragma unroll
-        for (int j = 0; j < LANES; ++j) tau = tau + fromLane<LANES>(term, j);
+            for (int j = 0; j < LANES; ++j) tau = tau + fromLane<LANES>(term, j);
+        }
     }
     if (!live || sub != 0) return;
     const float t = apart ? expf(-tau) : 1.0f;
     tr[(lz * p.ly + ly) * p.lx + lx] = t;
-    if (!(fabsf(t) <= 1e30f)) occ->irregular = 1u;
+    if (SKIP && !(fabsf(t) <= 1e30f)) occ->irregular = 1u;
 }
 
-__global__ void __launch_bounds__(128) cfgTransmittance(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ, ConfigParams p) {
+template <bool SKIP>
+__device__ __forceinline__ void cfgTransmittanceOwn(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ, const ConfigParams& p) {
     const int lx = blockIdx.x * blockDim.x + threadIdx.x;
     const int ly = blockIdx.y;
     const int lz = blockIdx.z;
     if (lx >= p.lx) return;
-    cfgTransmittanceAt<1>(tr, a, occ, p, lx, ly, lz, 0, true);
+    if (SKIP && occ->look == kCfgEvery) {  // (a copy of its own: in one loop with the cut the registers slow both)
+        cfgTransmittanceAt<1, false, true>(tr, a, occ, p, lx, ly, lz, 0, true);
+        return;
+    }
+    cfgTransmittanceAt<1, SKIP>(tr, a, occ, p, lx, ly, lz, 0, true);
 }
-
+template <bool SKIP>
+__device__ __forceinline__ void cfgTransmittanceShared(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ,
+                                                       const ConfigParams& p) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kRayLanes, row = i / p.lx;
+    cfgTransmittanceAt<kRayLanes, SKIP>(tr, a, occ, p, i - row * p.lx, row % p.ly, row / p.ly, threadIdx.x % kRayLanes,
+                                        i < p.lx * p.ly * p.lz);
+}
+__global__ void __launch_bounds__(128) cfgTransmittance(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ, ConfigParams p) {
+    cfgTransmittanceOwn<true>(tr, a, occ, p);
+}
+__global__ void __launch_bounds__(128) cfgTransmittanceEvery(float* __restrict__ tr, const Rec4* __restrict__ a, ConfigParams p) {
+    cfgTransmittanceOwn<false>(tr, a, nullptr, p);
+}
 __global__ void __launch_bounds__(128) cfgTransmittanceLanes(float* __restrict__ tr, const Rec4* __restrict__ a, CfgOccupancy* occ,
                                                              ConfigParams p) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kRayLanes, row = i / p.lx;
-    cfgTransmittanceAt<kRayLanes>(tr, a, occ, p, i - row * p.lx, row % p.ly, row / p.ly, threadIdx.x % kRayLanes, i < p.lx * p.ly * p.lz);
+    cfgTransmittanceShared<true>(tr, a, occ, p);
+}
+__global__ void __launch_bounds__(128) cfgTransmittanceLanesEvery(float* __restrict__ tr, const Rec4* __restrict__ a, ConfigParams p) {
+    cfgTransmittanceShared<false>(tr, a, nullptr, p);
 }
 
 // One pixel: the camera ray's chord through the grid box in primarySamples
 // midpoint samples; absorption, in-scattering of the point light (its
 // transmittance volume) and emission; a dark background behind.
-template <int LANES>
+template <int LANES, bool SKIP>
 __device__ __forceinline__ void cfgRaymarchAt(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
                                               const CfgOccupancy* __restrict__ occ, const ConfigParams& p, int px, int py, int sub, bool live) {
     const float sx = (2.0f * (static_cast<float>(px) + 0.5f) / static_cast<float>(p.frameW) - 1.0f) * p.tanHalf * p.aspect;
@@ -658,8 +717,9 @@ __device__ __forceinline__ void cfgRaymarchAt(float4* __restrict__ hdr, const Re
     }
     float r = 0.0f, g = 0.0f, b = 0.0f, view = 1.0f;
     const float ds = (t1 - t0) / static_cast<float>(p.primarySamples);
-    const bool skip = ds < 1e30f && fabsf(p.albedo * p.lightIntensity) <= 1e8f && occ->irregular == 0u;
-    const bool ask = skip && occ->dense == 0u;
+    const unsigned look = SKIP ? occ->look : static_cast<unsigned>(kCfgEvery);
+    const bool skip = look != kCfgEvery && ds < 1e30f && fabsf(p.albedo * p.lightIntensity) <= 1e8f && (!SKIP || occ->irregular == 0u);
+    const bool ask = skip && look == kCfgAsk;
     int first = 0, last = p.primarySamples;
     if (skip) samplesInBox(occ, p, eye, dir, t0, ds, p.primarySamples, first, last);
     hit = hit && t1 > t0;
@@ -724,21 +784,42 @@ __device__ __forceinline__ void cfgRaymarchAt(float4* __restrict__ hdr, const Re
     hdr[py * p.frameW + px] = make_float4(r + view * 0.015f, g + view * 0.016f, b + view * 0.020f, 1.0f - view);
 }
 
-__global__ void __launch_bounds__(128) cfgRaymarch(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
-                                                   const CfgOccupancy* __restrict__ occ, ConfigParams p) {
+template <bool SKIP>
+__device__ __forceinline__ void cfgRaymarchOwn(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
+                                               const CfgOccupancy* __restrict__ occ, const ConfigParams& p) {
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
     const int py = blockIdx.y * blockDim.y + threadIdx.y;
     if (px >= p.frameW || py >= p.frameH) return;
-    cfgRaymarchAt<1>(hdr, a, tr, occ, p, px, py, 0, true);
+    if (SKIP && occ->look == kCfgEvery) {
+        cfgRaymarchAt<1, false>(hdr, a, tr, occ, p, px, py, 0, true);
+        return;
+    }
+    cfgRaymarchAt<1, SKIP>(hdr, a, tr, occ, p, px, py, 0, true);
 }
-
 // A warp's rays are 4 x 2 pixels, a block's 16 x 2.
-__global__ void __launch_bounds__(128) cfgRaymarchLanes(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
-                                                        const CfgOccupancy* __restrict__ occ, ConfigParams p) {
+template <bool SKIP>
+__device__ __forceinline__ void cfgRaymarchShared(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
+                                                  const CfgOccupancy* __restrict__ occ, const ConfigParams& p) {
     const int ray = (threadIdx.x & 31) / kRayLanes, warp = threadIdx.x >> 5;
     const int px = blockIdx.x * 16 + warp * 4 + (ray & 3);
     const int py = blockIdx.y * 2 + (ray >> 2);
-    cfgRaymarchAt<kRayLanes>(hdr, a, tr, occ, p, px, py, threadIdx.x % kRayLanes, px < p.frameW && py < p.frameH);
+    cfgRaymarchAt<kRayLanes, SKIP>(hdr, a, tr, occ, p, px, py, threadIdx.x % kRayLanes, px < p.frameW && py < p.frameH);
+}
+__global__ void __launch_bounds__(128) cfgRaymarch(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
+                                                   const CfgOccupancy* __restrict__ occ, ConfigParams p) {
+    cfgRaymarchOwn<true>(hdr, a, tr, occ, p);
+}
+__global__ void __launch_bounds__(128) cfgRaymarchEvery(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
+                                                        ConfigParams p) {
+    cfgRaymarchOwn<false>(hdr, a, tr, nullptr, p);
+}
+__global__ void __launch_bounds__(128) cfgRaymarchLanes(float4* __restrict__ hdr, const Rec4* __restrict__ a, const float* __restrict__ tr,
+                                                        const CfgOccupancy* __restrict__ occ, ConfigParams p) {
+    cfgRaymarchShared<true>(hdr, a, tr, occ, p);
+}
+__global__ void __launch_bounds__(128) cfgRaymarchLanesEvery(float4* __restrict__ hdr, const Rec4* __restrict__ a,
+                                                             const float* __restrict__ tr, ConfigParams p) {
+    cfgRaymarchShared<false>(hdr, a, tr, nullptr, p);
 }
 
 // ---- the incremental projection of the multigrid solve (fire_mg.cu) ----
@@ -937,7 +1018,7 @@ __global__ void __launch_bounds__(kBatchThreads) batchOccupancy(const BatchScene
             w = 32;
             h = 1 << 30;
         },
-        [](const BatchScene& B, int, int lane, int unit, int) { cfgOccupancyAt(B.occupancy, B.aOut, nullptr, B.c, unit, lane); });
+        [](const BatchScene& B, int, int lane, int unit, int) { cfgOccupancyAt(B.occupancy, B.aOut, nullptr, B.c, unit, 1 << 30, lane); });
 }
 
 __global__ void __launch_bounds__(kBatchThreads) batchTransmittance(const BatchScene* __restrict__ scenes, const BatchPlan* __restrict__ plan) {
@@ -947,7 +1028,7 @@ __global__ void __launch_bounds__(kBatchThreads) batchTransmittance(const BatchS
             w = B.c.lx;
             h = B.c.ly;
         },
-        [](const BatchScene& B, int, int x, int y, int z) { cfgTransmittanceAt<1>(B.transmittance, B.aOut, B.occupancy, B.c, x, y, z, 0, true); });
+        [](const BatchScene& B, int, int x, int y, int z) { cfgTransmittanceAt<1, true>(B.transmittance, B.aOut, B.occupancy, B.c, x, y, z, 0, true); });
 }
 
 __global__ void __launch_bounds__(kBatchThreads) batchRaymarch(const BatchScene* __restrict__ scenes, const BatchPlan* __restrict__ plan) {
@@ -957,7 +1038,7 @@ __global__ void __launch_bounds__(kBatchThreads) batchRaymarch(const BatchScene*
             w = B.c.frameW;
             h = B.c.frameH;
         },
-        [](const BatchScene& B, int, int x, int y, int) { cfgRaymarchAt<1>(B.hdr, B.aOut, B.transmittance, B.occupancy, B.c, x, y, 0, true); });
+        [](const BatchScene& B, int, int x, int y, int) { cfgRaymarchAt<1, true>(B.hdr, B.aOut, B.transmittance, B.occupancy, B.c, x, y, 0, true); });
 }
 
 __global__ void __launch_bounds__(kBatchThreads) batchPackHdr(const BatchScene* __restrict__ scenes, const BatchPlan* __restrict__ plan) {

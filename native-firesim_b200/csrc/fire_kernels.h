@@ -216,28 +216,39 @@ __global__ void cfgApplyForces(FaceT* uOut, FaceT* vOut, FaceT* wOut, Velocity v
 // fuel or soot is not zero in any cell that a sample whose first corner lies in
 // the brick reads.  box is the bounding box of the set bricks: 2^20 - lo and
 // hi + 1 per axis, so that zero is empty.  irregular: some transmittance is not
-// within +-1e30, so that a sample of nothing need not add nothing.  dense: half
-// of the bricks or more are set.  done and the acc fields are the build's own,
+// within +-1e30, so that a sample of nothing need not add nothing.  look: what
+// the rays take from it (CfgLook).  done and the acc fields are the build's own,
 // zero between builds.
+enum CfgLook : unsigned {
+    kCfgAsk = 0,    // a sample in the box asks for its brick
+    kCfgBox = 1,    // half of the bricks or more are set: every sample in the box
+    kCfgEvery = 2,  // the grid is largely full: every sample (no box and no flags are built)
+};
 struct CfgOccupancy {
-    unsigned done, accIrregular, irregular, accSet, dense, unused[3];
+    unsigned done, accIrregular, irregular, accSet, look, unused[3];
     unsigned acc[6], box[6];
 };
 __host__ __device__ inline int cfgBricks(int n) { return (n + 3) >> 2; }
 inline size_t cfgOccupancyBytes(int nx, int ny, int nz) {
     return sizeof(CfgOccupancy) + static_cast<size_t>(cfgBricks(nx)) * cfgBricks(ny) * cfgBricks(nz);
 }
-// A warp builds seven bricks along x (lane 28 reads the cells that the last one
+// A warp builds seven bricks along x at a time (lane 28 reads the cells that the last one
 // shares with the next).
 __host__ __device__ inline int cfgOccupancyUnits(int nx, int ny, int nz) {
     return ((cfgBricks(nx) + 6) / 7) * cfgBricks(ny) * cfgBricks(nz);
 }
+constexpr int kOccupancyBlocks = 148 * 8;  // of 4 warps, at most: they stay on the chip, and the build's end counts warps
 __global__ void cfgOccupancyBuild(CfgOccupancy* occ, const Rec4* a, const float* tr, ConfigParams p);
 constexpr int kRayLanes = 4;  // lanes of a ray in the Lanes kernels
+// With an occupancy, or without one for every sample.
 __global__ void cfgTransmittance(float* tr, const Rec4* a, CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgTransmittanceEvery(float* tr, const Rec4* a, ConfigParams p);
 __global__ void cfgTransmittanceLanes(float* tr, const Rec4* a, CfgOccupancy* occ, ConfigParams p);
-__global__ void cfgRaymarchLanes(float4* hdr, const Rec4* a, const float* tr, const CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgTransmittanceLanesEvery(float* tr, const Rec4* a, ConfigParams p);
 __global__ void cfgRaymarch(float4* hdr, const Rec4* a, const float* tr, const CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgRaymarchEvery(float4* hdr, const Rec4* a, const float* tr, ConfigParams p);
+__global__ void cfgRaymarchLanes(float4* hdr, const Rec4* a, const float* tr, const CfgOccupancy* occ, ConfigParams p);
+__global__ void cfgRaymarchLanesEvery(float4* hdr, const Rec4* a, const float* tr, ConfigParams p);
 
 // ---------------------------------------------------------------------------
 // Multigrid pressure solve of the config physics (fire_mg.cu): the

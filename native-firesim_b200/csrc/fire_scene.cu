@@ -1859,6 +1859,19 @@ bool Scene::ensureConfigBuffers(std::string& err) {
            check("clear config transmittance", cudaMemsetAsync(cfgLight_, 0, bytes, stream), err);
 }
 
+namespace {
+long long pixelSamples(const ConfigParams& c) { return static_cast<long long>(c.frameW) * c.frameH * c.primarySamples; }
+}  // namespace
+
+// The occupancy for rays of that many samples in all (about 80 a nanosecond), or
+// null where its build could cost more than it saves.  It takes 4 us on a grid
+// that is largely full, as long as 300,000 samples, at most a sixteenth of what it
+// is built for; otherwise it reads every cell (65 us at 256^3, a quarter of a
+// sample each) and saves the samples of the empty part.
+CfgOccupancy* Scene::cfgOccupancyFor(long long samples) const {
+    return samples >= 4800000 + static_cast<long long>(cells_) / 2 ? cfgOcc_ : nullptr;
+}
+
 // One step of this scene inside a FireBatch: the frame's bookkeeping (clocks,
 // reset, frame index), the buffers the batched kernels need, and the
 // descriptor of this step's buffers; then the host state advances as the
@@ -1950,13 +1963,21 @@ bool Scene::prepareBatched(std::string& err) {
     return cfgNoise_ != nullptr || alloc(reinterpret_cast<void**>(&cfgNoise_), cells_ * sizeof(float4), "cudaMalloc config noise field", err);
 }
 
-// Rays up to which a light or camera ray gets kRayLanes lanes instead of one.
-// Four lanes fill the chip and shorten a ray's chain of dependent loads; past a
-// warp or so per scheduler slot their shuffles and idle lanes cost more.  Dense
-// grids, light + render: 24^3 at 64x64 97 -> 44 us, 61x47x83 at 320x180 124 -> 79,
-// 64^3 at 256x256 179 -> 144 (65,536 camera and 32,768 light rays); 128^3 at
-// 512x512 (262,144 of each) 587 -> 638, 256^3 1,601 -> 1,945.
-constexpr long long kLaneRays = 131072;
+// Where a light or camera ray gets kRayLanes lanes instead of one.  Four lanes
+// fill the chip and shorten a ray's chain of dependent loads; past that their
+// shuffles and idle lanes cost more.  Light, 48 samples a ray, one lane and four:
+// 4,096 rays 19.5 and 13.3 us, 21,952 23.5 and 23.5, 32,768 27.6 and 25.6, 46,656
+// 35.8 and 35.8, 64,000 46 and 50.  Camera, full grids: 36,864 rays of 32 samples
+// 35.8 and 27.6 us (48^3), 65,536 of 32 37.9 and 43.9, of 128 128 and 103; of 96 in
+// 192^3, whose records exceed what the L2 holds beside them, 138 and 155 (with
+// most of it empty 105 and 76).
+namespace {
+constexpr long long kLightLaneRays = 32768;
+bool pixelLanes(const ConfigParams& c, size_t cells, bool skips) {
+    const long long rays = static_cast<long long>(c.frameW) * c.frameH;
+    return rays <= 36864 || (rays <= std::min(131072LL, 1024LL * c.primarySamples) && (skips || cells <= 4000000));
+}
+}  // namespace
 
 // The config physics on the frame's stage ids: advect velocity, advect +
 // react + emit, forces (vorticity, cell accelerations, faces with the walls),
@@ -1970,7 +1991,8 @@ bool Scene::runConfigStages(int first, int last, const FrameParams& p, std::stri
     // Built by this call's light stage from the records that its render stage
     // reads (the stages that write them come earlier); a call that renders
     // without it, maybe after the caller has set fields, builds its own.
-    bool occupancyBuilt = false;
+    // A light pass or render without one takes every sample.
+    const CfgOccupancy* built = nullptr;
     for (int s = first; s <= last; ++s) {
         const ConfigParams c = configParams();
         switch (s) {
@@ -2039,25 +2061,48 @@ bool Scene::runConfigStages(int first, int last, const FrameParams& p, std::stri
                 break;
             case kLightBuild: {
                 const int lbx = rowThreads(cfgLx_);
-                cfgOccupancyBuild<<<(cfgOccupancyUnits(nx, ny, nz) + 3) / 4, 128, 0, stream>>>(cfgOcc_, sa_[cur_], nullptr, c); ++launches_;
-                occupancyBuilt = true;
                 const long long rays = static_cast<long long>(cfgLx_) * cfgLy_ * cfgLz_;
-                if (rays <= kLaneRays) {
-                    cfgTransmittanceLanes<<<static_cast<int>((rays * kRayLanes + 127) / 128), 128, 0, stream>>>(cfgLight_, sa_[cur_], cfgOcc_, c); ++launches_;
-                } else {
-                    cfgTransmittance<<<dim3((cfgLx_ + lbx - 1) / lbx, cfgLy_, cfgLz_), lbx, 0, stream>>>(cfgLight_, sa_[cur_], cfgOcc_, c); ++launches_;
+                CfgOccupancy* occ = cfgOccupancyFor(rays * c.lightSamples + (last >= kRender ? pixelSamples(c) : 0));
+                if (occ != nullptr) {
+                    cfgOccupancyBuild<<<std::min((cfgOccupancyUnits(nx, ny, nz) + 3) / 4, kOccupancyBlocks), 128, 0, stream>>>(occ, sa_[cur_], nullptr, c); ++launches_;
                 }
+                built = occ;
+                const int laneBlocks = static_cast<int>((rays * kRayLanes + 127) / 128);
+                const dim3 blocks((cfgLx_ + lbx - 1) / lbx, cfgLy_, cfgLz_);
+                if (rays <= kLightLaneRays) {
+                    if (occ != nullptr) {
+                        cfgTransmittanceLanes<<<laneBlocks, 128, 0, stream>>>(cfgLight_, sa_[cur_], occ, c);
+                    } else {
+                        cfgTransmittanceLanesEvery<<<laneBlocks, 128, 0, stream>>>(cfgLight_, sa_[cur_], c);
+                    }
+                } else if (occ != nullptr) {
+                    cfgTransmittance<<<blocks, lbx, 0, stream>>>(cfgLight_, sa_[cur_], occ, c);
+                } else {
+                    cfgTransmittanceEvery<<<blocks, lbx, 0, stream>>>(cfgLight_, sa_[cur_], c);
+                }
+                ++launches_;
                 break;
             }
             case kRender:
-                if (!occupancyBuilt) {
-                    cfgOccupancyBuild<<<(cfgOccupancyUnits(nx, ny, nz) + 3) / 4, 128, 0, stream>>>(cfgOcc_, sa_[cur_], cfgLight_, c); ++launches_;
+                if (first > kLightBuild) {
+                    CfgOccupancy* occ = cfgOccupancyFor(pixelSamples(c));
+                    if (occ != nullptr) {
+                        cfgOccupancyBuild<<<std::min((cfgOccupancyUnits(nx, ny, nz) + 3) / 4, kOccupancyBlocks), 128, 0, stream>>>(occ, sa_[cur_], cfgLight_, c); ++launches_;
+                    }
+                    built = occ;
                 }
-                if (static_cast<long long>(frameW) * frameH <= kLaneRays) {
-                    cfgRaymarchLanes<<<dim3((frameW + 15) / 16, (frameH + 1) / 2), 128, 0, stream>>>(hdr_, sa_[cur_], cfgLight_, cfgOcc_, c); ++launches_;
+                if (const dim3 lanes((frameW + 15) / 16, (frameH + 1) / 2), own((frameW + 15) / 16, (frameH + 7) / 8); pixelLanes(c, cells_, built != nullptr)) {
+                    if (built != nullptr) {
+                        cfgRaymarchLanes<<<lanes, 128, 0, stream>>>(hdr_, sa_[cur_], cfgLight_, built, c);
+                    } else {
+                        cfgRaymarchLanesEvery<<<lanes, 128, 0, stream>>>(hdr_, sa_[cur_], cfgLight_, c);
+                    }
+                } else if (built != nullptr) {
+                    cfgRaymarch<<<own, dim3(16, 8), 0, stream>>>(hdr_, sa_[cur_], cfgLight_, built, c);
                 } else {
-                    cfgRaymarch<<<dim3((frameW + 15) / 16, (frameH + 7) / 8), dim3(16, 8), 0, stream>>>(hdr_, sa_[cur_], cfgLight_, cfgOcc_, c); ++launches_;
+                    cfgRaymarchEvery<<<own, dim3(16, 8), 0, stream>>>(hdr_, sa_[cur_], cfgLight_, c);
                 }
+                ++launches_;
                 break;
             case kTonemap:
                 tonemapOverlay<<<dim3((frameW + 15) / 16, (frameH + 15) / 16), dim3(16, 16), 0, stream>>>(bgra_, hdr_, p, 1, 0); ++launches_;

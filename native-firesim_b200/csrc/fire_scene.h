@@ -253,6 +253,7 @@ private:
     FirePhysicsParams physics_{};
     float4* cfgVort_ = nullptr;   // vorticity (x, y, z, |omega|) per cell, allocated on first use
     float* cfgLight_ = nullptr;   // transmittance to the point light, half resolution
+    CfgOccupancy* cfgOccupancyFor(long long samples) const;
     CfgOccupancy* cfgOcc_ = nullptr;  // which bricks hold something to see (in cfgLight_'s allocation, behind it)
     float4* cfgNoise_ = nullptr;  // curl-noise acceleration per cell, rebuilt when its parameters change
     bool cfgNoiseValid_ = false;
