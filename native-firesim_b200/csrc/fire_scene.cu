@@ -1072,73 +1072,94 @@ bool Scene::sourceLattice(const FrameParams& p, HashLattice2& l) const {
     return fits;
 }
 
-// The tables of the raymarch's noise fields for this frame: per field and
-// octave every lattice cell that a sample position in [0, 1]^3 can reach, one
-// cell wider on each side (a cell outside is hashed in place, so the margin
-// affects speed only; an octave beyond kLatticeReach has no table).  The room
-// does not depend on the time (1.46 M entries).
-// They lie in the force scratch, which no stage of a frame uses, where the grid
-// has that many cells; else in a buffer that the first frame allocates, and a
-// frame goes without where that fails or the stream is being captured.
-// The finest octave of the finest field has no table: its 7 M cells are 111 MB
-// more per scene, and hashing them costs what they save (render with and
-// without it: 0.56 against 0.49 ms at 128x128, 1.21 against 1.25 ms at
-// 512x512, 2.19 against 2.32 ms at 1280x720).  Its second octave, 15 MB, pays
-// at every size (1.31 -> 1.25 ms at 512x512).
+namespace {
+
+// The raymarch's noise fields: their spans over the unit cube and the octave step.
+constexpr double kRenderSpan[4][3] = {{7.0, 5.0, 9.0}, {8.0, 8.0, 6.0}, {42.0, 54.0, 43.0}, {15.0, 13.0, 17.0}};
+constexpr double kRenderScale[3] = {2.03, 2.01, 2.07}, kRenderShift[3] = {17.7, -9.2, 5.1};
+
+// Entries of field f's octave o along axis d: every lattice cell that a sample
+// position in [0, 1]^3 can reach, one cell wider on each side (a cell outside is
+// hashed in place, so the margin affects speed only).  They do not depend on the
+// time.  The finest octave of the finest field has no table: its 7 M cells are
+// 111 MB more per scene, and hashing them costs what they save (render with and
+// without it: 0.56 against 0.49 ms at 128x128, 1.21 against 1.25 ms at 512x512,
+// 2.19 against 2.32 ms at 1280x720).  Its second octave, 15 MB, pays at every size
+// (1.31 -> 1.25 ms at 512x512).
+int renderTableSize(int f, int o, int d) {
+    if (f == 2 && o + 1 == kRenderOctaves) return 0;
+    return static_cast<int>(std::ceil(kRenderSpan[f][d] * std::pow(kRenderScale[d], o))) + 3 + (d == 2 ? 1 : 0);
+}
+
+// Entries of all tables (1.46 M).
+size_t renderNoiseEntries() {
+    size_t total = 0;
+    for (int k = 0; k < kRenderTables; ++k) {
+        const int f = k / kRenderOctaves, o = k % kRenderOctaves;
+        total += static_cast<size_t>(renderTableSize(f, o, 0)) * renderTableSize(f, o, 1) * renderTableSize(f, o, 2);
+    }
+    return total;
+}
+
+}  // namespace
+
+// The tables of the raymarch's noise fields for this frame; an octave beyond
+// kLatticeReach has none.  They lie in the force scratch, which no stage of a
+// frame uses, where the grid has the cells for them, else in renderNoise_.
 bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
-    if (!latticesEnabled_ || renderNoiseRefused_) return false;
+    float4* room = cells_ >= renderNoiseEntries() ? contrib_ : renderNoise_;
+    if (!latticesEnabled_ || room == nullptr) return false;
     const double t = p.time;
     const double lo[4][3] = {{t * 0.18, -t * 0.11, t * 0.07}, {-t * 0.14, t * 0.10, -t * 0.08}, {t * 0.72, -t * 1.28, t * 0.38},
                              {-t * 0.72, -t * 1.08, t * 0.32}};
-    const double span[4][3] = {{7.0, 5.0, 9.0}, {8.0, 8.0, 6.0}, {42.0, 54.0, 43.0}, {15.0, 13.0, 17.0}};
-    const double scale[3] = {2.03, 2.01, 2.07}, shift[3] = {17.7, -9.2, 5.1};
-    int total = 0, capacity = 0;
+    n.values = room;
+    n.total = 0;
     for (int f = 0; f < 4; ++f) {
-        double a[3] = {lo[f][0], lo[f][1], lo[f][2]}, w[3] = {span[f][0], span[f][1], span[f][2]};
+        double a[3] = {lo[f][0], lo[f][1], lo[f][2]};
         for (int o = 0; o < kRenderOctaves; ++o) {
             const int k = f * kRenderOctaves + o;
-            int org[3], size[3];
-            bool within = true;
+            const bool within = withinReach(a[0]) && withinReach(a[1]) && withinReach(a[2]);
+            int origin[3], size[3];
             for (int d = 0; d < 3; ++d) {
-                within = within && withinReach(a[d]);
-                org[d] = within ? static_cast<int>(std::floor(a[d])) - 1 : 0;
-                size[d] = static_cast<int>(std::ceil(w[d])) + 3 + (d == 2 ? 1 : 0);
-                a[d] = a[d] * scale[d] + shift[d];
-                w[d] *= scale[d];
+                origin[d] = within ? static_cast<int>(std::floor(a[d])) - 1 : 0;
+                size[d] = within ? renderTableSize(f, o, d) : 0;
+                a[d] = a[d] * kRenderScale[d] + kRenderShift[d];
             }
-            const bool room = f != 2 || o + 1 < kRenderOctaves, table = room && within;
-            n.ox[k] = org[0];
-            n.oy[k] = org[1];
-            n.oz[k] = org[2];
-            n.sx[k] = table ? size[0] : 0;
-            n.sy[k] = table ? size[1] : 0;
-            n.sz[k] = table ? size[2] : 0;
-            n.offset[k] = total;
-            total += n.sx[k] * n.sy[k] * n.sz[k];
-            capacity += room ? size[0] * size[1] * size[2] : 0;
+            n.ox[k] = origin[0];
+            n.oy[k] = origin[1];
+            n.oz[k] = origin[2];
+            n.sx[k] = size[0];
+            n.sy[k] = size[1];
+            n.sz[k] = size[2];
+            n.offset[k] = n.total;
+            n.total += size[0] * size[1] * size[2];
         }
     }
-    if (cells_ >= static_cast<size_t>(capacity)) {
-        n.values = contrib_;
-        n.total = total;
-        return true;
+    return true;
+}
+
+void Scene::placeRenderNoise() {
+    const bool wanted = physics_.mode == 0 && cells_ < renderNoiseEntries();
+    if (wanted == (renderNoise_ != nullptr) || (wanted && renderNoiseRefused_)) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaSetDevice(device) != cudaSuccess || cudaStreamIsCapturing(stream, &capture) != cudaSuccess ||
+        capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
     }
-    if (renderNoise_ == nullptr) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return false;
-        }
+    const size_t bytes = renderNoiseEntries() * sizeof(float4);
+    if (wanted) {
         std::string ignored;
-        if (!alloc(reinterpret_cast<void**>(&renderNoise_), static_cast<size_t>(capacity) * sizeof(float4), "cudaMalloc render noise", ignored)) {
+        if (!alloc(reinterpret_cast<void**>(&renderNoise_), bytes, "cudaMalloc render noise", ignored)) {
             cudaGetLastError();
             renderNoiseRefused_ = true;
-            return false;
         }
+        return;
     }
-    n.values = renderNoise_;
-    n.total = total;
-    return true;
+    cudaStreamSynchronize(stream);  // frames that read them may be queued
+    deviceFree(renderNoise_);
+    renderNoise_ = nullptr;
+    deviceBytes_ -= bytes;
 }
 
 bool Scene::runStages(int first, int last, const FrameParams& p, std::string& err) {

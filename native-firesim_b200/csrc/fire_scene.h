@@ -141,6 +141,11 @@ public:
     // Physics of the following passes (mode 0 reference, mode 1 config physics).
     bool setPhysics(const FirePhysicsParams& params, std::string& err);
     const FirePhysicsParams& physics() const { return physics_; }
+    // Gives a scene of the reference physics the room for its noise tables, and
+    // takes it from one of the config physics, which has none.  Whoever makes the
+    // scene or sets its physics calls this, so that no frame allocates and
+    // deviceBytes() has it beforehand; a scene without the room hashes in place.
+    void placeRenderNoise();
     // Steps of the config physics since the last reset (the emitter jitter's counter).
     unsigned long long configStep() const { return cfgStep_; }
     bool synchronize(std::string& err);
@@ -221,11 +226,12 @@ private:
     bool sourceLattice(const FrameParams& p, HashLattice2& l) const;
     float* sourceLattice_ = nullptr;
     size_t sourceCapacity_ = 0;
-    // Raymarch work list: tile order (centre first) and the tile counter.
-    // Hash tables of the raymarch's noise fields, allocated by the first frame that uses them.
+    // Hash tables of the raymarch's noise fields, where the force scratch has no room
+    // for them (placeRenderNoise); null: frames hash in place.
     bool renderNoise(const FrameParams& p, RenderNoise& n);
     float4* renderNoise_ = nullptr;
-    bool renderNoiseRefused_ = false;  // their allocation failed: frames hash in place
+    bool renderNoiseRefused_ = false;  // their allocation failed
+    // Raymarch work list: tile order (centre first) and the tile counter.
     int* rayTileOrder_ = nullptr;
     int* rayTileCounter_ = nullptr;
     int rayTilesX_ = 0, rayTileCount_ = 0;

@@ -68,6 +68,7 @@ extern "C" FireScene* fireSceneCreate(int device, int frameW, int frameH, int nx
         fail(err);
         return nullptr;
     }
+    scene->placeRenderNoise();
     FireScene* h = new FireScene;
     h->scene = std::move(scene);
     h->device = device;
@@ -101,6 +102,7 @@ extern "C" bool fireSceneSetPhysicsParams(FireScene* scene, const FirePhysicsPar
     if (params == nullptr) return fail("Physics parameter pointer was null.");
     std::string err;
     if (!scene->scene->setPhysics(*params, err)) return fail(err);
+    scene->scene->placeRenderNoise();
     return true;
 }
 
@@ -666,6 +668,10 @@ extern "C" bool fireServerRun(FireServer* server, double maxSeconds, FireServeRe
                     ok = fail(err);
                     break;
                 }
+                // The noise tables of a scene that renders the reference physics, before it is
+                // counted: no frame allocates.  (A pooled scene that was made for another
+                // request may be without them and hashes in place.)
+                if (r.physics.mode == 0 && r.renderEvery > 0) a->scene->placeRenderNoise();
                 a->bytes = a->scene->deviceBytes() + frameBytes(r);
                 server->bytesByShape[shape] = a->bytes;
                 if (inUse + a->bytes > server->budget && !active.empty()) {

@@ -1,0 +1,59 @@
+"""The raymarch's noise tables are part of a scene from its making on (needs a
+GPU): no frame changes what a scene holds, a served scene is counted with them
+before it is admitted, and the config physics, which has none, gives them back."""
+from __future__ import annotations
+
+import pytest
+
+from test_gpu_serving import _request
+
+pytestmark = pytest.mark.gpu
+
+DIMS = (32, 28, 24)
+
+
+def _frame(pkg, abi, scene, hdr, reset):
+    scene.set_hdr_buffer(hdr.data_ptr(), 64 * 16, 0)
+    s = abi.validation_settings(0, width=64, height=48)
+    s.reset = reset
+    scene.step(s, render=True)
+    scene.synchronize()
+
+
+def test_no_frame_changes_what_a_scene_holds(pkg, abi):
+    import torch
+
+    hdr = torch.zeros((48, 64, 4), device="cuda")
+    scene = pkg.Scene(64, 48, *DIMS)
+    made = scene.device_bytes()
+    _frame(pkg, abi, scene, hdr, 1)
+    assert scene.device_bytes() == made
+    p = abi.default_physics(*DIMS)
+    p.mode = 1
+    scene.set_physics(p)
+    without = scene.device_bytes()
+    assert made - without > 20_000_000
+    p.mode = 0
+    scene.set_physics(p)
+    assert scene.device_bytes() == made
+    _frame(pkg, abi, scene, hdr, 1)
+    assert scene.device_bytes() == made
+    scene.close()
+
+
+def test_server_counts_a_scene_as_it_is_after_a_frame(pkg, abi):
+    import torch
+
+    hdr = torch.zeros((48, 64, 4), device="cuda")
+    scene = pkg.Scene(64, 48, *DIMS)
+    _frame(pkg, abi, scene, hdr, 1)
+    rendered = scene.device_bytes() + 64 * 48 * 16
+    scene.close()
+    server = pkg.Server(budget_bytes=int(2.5 * rendered))
+    for i in range(4):
+        server.submit(_request(abi, i, DIMS, steps=6, arrival=0.0, scene=0, render_every=2))
+    rep = server.run(60.0)
+    server.close()
+    assert rep["completed"] == 4
+    assert rep["admittedPeak"] <= 2
+    assert rep["deviceBytesPeak"] == rep["admittedPeak"] * rendered
