@@ -253,7 +253,7 @@ FIRE_API bool fireCudaGetLaunchCount(unsigned long long* count);
  *
  * Limit: at most 1,048,576 cells (nx*ny*nz); larger grids are rejected.  The
  * per-cell increments live in one fixed 16 MiB array, and the curl noise's hash
- * lattices in one of 0.9 MiB, that every GPU loading the library holds until
+ * lattices in one of 0.84 MiB, that every GPU loading the library holds until
  * exit.  The first call on each device resolves their device addresses, so make
  * it before any stream capture.  All calls share the arrays: calls that overlap
  * on the GPU (other streams, other host threads) race.  Each call overwrites

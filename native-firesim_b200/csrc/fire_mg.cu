@@ -41,7 +41,12 @@
 // kMgTailCells cells down) is solved by one CTA in shared memory (in its
 // global buffers if it does not fit, as for a grid that cannot coarsen).  Reads of
 // data written inside the launch go through L2 (ld.global.cg), as L1 is not
-// coherent between SMs.
+// coherent between SMs; all but the coarse correction that a tile copies into
+// shared memory by cp.async, which passes through L1 (cells of 4 bytes have no
+// other form).  Its lines may not be older than the last grid barrier: thread 0's
+// ld.acquire there, and the __syncthreads after it, order every later read of the
+// CTA behind the other CTAs' writes.  A barrier that polled with relaxed loads
+// would need a fence for it.
 //
 // Compiled with -fmad=false: every operation rounds as written, so a CPU
 // restatement in the same order gives the same bits, and a scene gives the
@@ -517,25 +522,20 @@ __device__ __forceinline__ float quadSum(const MgLevel& L, const Quad& q, int e,
 }
 
 // ---- smoothing: up to four half sweeps of one tile in shared memory -------
-// A half sweep over global memory reads p (with its neighbours) and the rhs and
-// writes p through L2 for two flops a byte, and costs a grid barrier: 8.7 us at
-// 128^3 (of it 2.3 us of barrier), 45 us at 256^3, 3.8 us (2.1) at 32^3.  Four of
-// them as one phase of tiles take 24.5, 169 and 5.7 us; a tile of 32x16x16 cells
-// 2.9 us to load, 5.7 us for its four half sweeps (shared memory: 5.8 updates per
-// wavefront) and 0.7 us to store.  A V-cycle went 208 -> 169 us at 128^3, 711 ->
-// 671 us at 256^3 and 119 -> 93 us at 64^3.
-//
-// The transfers between levels run on the loaded tiles too: the correction is
-// interpolated into the tile before the post-smoothing (2 us a tile of 32x16x16,
-// where a phase over global memory took 12 us at 128^3, 75 us at 256^3, 4.5 us
-// at 32^3, 2 us of it barrier), the residual averaged from it after a
-// pre-smoothing whose last pass leaves the cells beside the tile valid (1.9 us a
-// tile; 8, 50 and 4.5 us).  With it a thread that has no column prepares the next
-// tile's operands.  A V-cycle went 169 -> 147 us at 128^3, 671 -> 635 us at 256^3
-// and 93 -> 80 us at 64^3.  The tile's stages are functions of their own: inlined
-// into one, or with the load and the interpolation in one, they spill, and a
-// cycle takes 160-240 us at 128^3; the phases over global memory, the other way
-// round, are slower as functions (175 us).
+// Over global memory a half sweep moves p and the rhs through L2 for two flops a
+// byte and costs a grid barrier: 8.7 us at 128^3 (2.3 of it barrier), 45 us at
+// 256^3, 3.8 us (2.1) at 32^3; four of them as one phase of tiles take 24.5, 169
+// and 5.7 us.  The transfers between levels run on the loaded tiles too: the
+// correction is interpolated into the tile before the post-smoothing, the residual
+// averaged from it after a pre-smoothing whose last pass leaves the cells beside
+// the tile valid (as phases of their own 12 and 8 us at 128^3, 75 and 50 at 256^3).
+// Per tile of 32x16x16 cells: load 2.9 us from L2, correction 2.1, four half sweeps
+// 5.7 (shared memory: 5.8 updates per wavefront), restriction 1.9, store 0.7.  A
+// V-cycle takes 147 us at 128^3 and 80 us at 64^3, where it took 208 and 119.
+// The tile's stages are functions of their own: inlined into one, or with the load
+// and the interpolation in one, they spill, and a cycle takes 160-240 us at 128^3;
+// the phases over global memory, the other way round, are slower as functions
+// (175 us).
 //
 // A CTA loads a tile of p and the rhs with a halo of four cells, runs `count`
 // half sweeps on it (each valid one cell less far into the halo) and writes the
@@ -954,9 +954,10 @@ __device__ __forceinline__ void flatCoords(const MgLevel& L, int i, int& x, int&
 
 }  // namespace
 
-// The persistent batched solve (see the file comment).  Work items of the
-// grid levels are units of one level of one scene (128 cells in memory order,
-// a quad per lane, where the row length is a multiple of 4; else chunks of
+// The persistent batched solve (see the file comment).  The grid levels' smoothing
+// takes one tile of one scene per CTA at a time, with the transfers that run on
+// it; the other transfers and the first phase take units (128 cells in memory
+// order, a quad per lane, where the row length is a multiple of 4; else chunks of
 // one row), one warp per unit; the tail is one CTA per scene; the residual is
 // one warp per chunk (mgResidualChunks); every CTA decides convergence from
 // the per-scene maxima, and one CTA per scene writes its gate record at the

@@ -24,7 +24,7 @@ namespace {
 // cells: 16 MiB, held by every GPU that loads the library until the process exits.
 constexpr int kNoAllocMaxCells = 1 << 20;
 static __device__ __align__(256) float4 g_forceScratch[kNoAllocMaxCells];
-// The curl noise's hash lattices of one call (0.8 MiB): every call that uses them
+// The curl noise's hash lattices of one call (0.84 MiB): every call that uses them
 // builds them before reading them.
 static __device__ __align__(256) float g_curlLattice[2 * firesim::kCurlLatticeEntries];
 

@@ -830,13 +830,17 @@ bool MgSolver::plan(int device, const std::vector<MgScene>& scenes, int maxCycle
     }
     // The smoothing's tile of each grid level: of the shapes the one whose waves
     // of tiles (a tile per CTA) take the least time, as a fixed latency of 1.5 us
-    // plus a time per cell of the region (measured: 9.3 us for 32x16x16's 23,040).
-    // Large tiles waste the least on halos; where they would leave SMs idle or
-    // end in a nearly empty wave, smaller ones finish sooner (32^3: 8x8x4 3.6 us).
-    // Beside a tail in global buffers the largest is left out: its shared memory
-    // (197 KB of the SM's 256 with the L1) leaves that tail, nearly all of such a
-    // cycle, hardly any L1 (250x198x154 34.7 ms a cycle with it, 22.9 without;
-    // 99x100x102 4.7 and 3.5 ms; the smaller shapes alone 22.9 and 3.5).
+    // plus a time per cell of the region (9.3 us for 32x16x16's 23,040; fitted to the
+    // half sweeps alone).  Large tiles waste the least on halos; where they would
+    // leave SMs idle or end in a nearly empty wave, smaller ones finish sooner (32^3:
+    // 8x8x4 3.6 us).  With the transfers on the tiles (14 to 17 us for 32x16x16) the
+    // choice holds: of 27 grids from 32^3 to 256^3, with each shape forced on level 0
+    // or 1, it was the fastest at 22 and within 1.4% at 4; at 176x208x128 32x16x16 on
+    // level 1 takes 232 instead of 240 us a cycle.
+    // Beside a tail in global buffers the largest is left out: its shared memory is
+    // 197 KB of the SM's 256 with the L1, where that tail's loads in flight land, and
+    // the tail is nearly all of such a cycle (250x198x154 34.7 ms a cycle with it,
+    // 22.9 without; 99x100x102 4.7 and 3.5 ms; with 16x8x8 as the largest the same).
     for (int l = 0; l < plan.gridLevels; ++l) {
         double best = 0.0;
         for (int k = globalTail ? 1 : 0; k < kMgTileShapes; ++k) {

@@ -26,13 +26,13 @@ struct HdrSlot {
     int format = 0;
 };
 
-// Inputs of the per-scene fuel-bed material table (fuelBedMaterial depends on nothing else).
 // The curl-noise lattices of the force pass at a time: their ranges and entry
 // counts (at most kCurlLatticeEntries each at any time that the table's margins
 // resolve), without storage.
 constexpr int kCurlLatticeEntries = 110592;
 void planCurlLattices(float time, HashLattice2& a, HashLattice2& b, int& na, int& nb);
 
+// Inputs of the per-scene fuel-bed material table (fuelBedMaterial depends on nothing else).
 struct MaterialKey {
     int sceneId = -1;
     float emitterRadius = 0.0f, emitterCenterX = 0.0f, emitterCenterZ = 0.0f;
