@@ -360,9 +360,9 @@ typedef struct FireScene FireScene;
 FIRE_API FireScene* fireSceneCreate(int device, int frameW, int frameH, int nx, int ny, int nz);
 /* Waits for the scene's queued work and frees it. */
 FIRE_API void fireSceneDestroy(FireScene* scene);
-/* Device memory the scene holds, in bytes (for admission against a budget).  A
- * scene of the reference physics with fewer than 1.46 M cells has 23 MB of noise
- * tables for its frames in it; setting the config physics gives them back. */
+/* Device memory the scene holds, in bytes (for admission against a budget).  For
+ * a scene of the reference physics with fewer than 1.46 M cells that is with the
+ * 23 MB of noise tables for its frames, which its first step allocates. */
 FIRE_API size_t fireSceneDeviceBytes(const FireScene* scene);
 FIRE_API bool fireSceneSetPressureSolver(FireScene* scene, int iterations, float omega);
 /* As fireCudaSetPressureTolerance / fireCudaSetPhysicsParams, for one scene. */

@@ -44,7 +44,6 @@ bool initialize(int frameW, int frameH, int nx, int ny, int nz) {
     if (!scene->reset(err)) {
         return fail(err);
     }
-    scene->placeRenderNoise();
     g_scene = std::move(scene);
     return true;
 }
@@ -245,7 +244,6 @@ bool fireCudaSetPhysicsParams(const FirePhysicsParams* params) {
     if (params == nullptr) return fail("Physics parameter pointer was null.");
     std::string err;
     if (!g_scene->setPhysics(*params, err)) return fail(err);
-    g_scene->placeRenderNoise();
     return true;
 }
 

@@ -1096,14 +1096,14 @@ int renderTableSize(int f, int o, int d) {
 }
 
 // Entries of all tables (1.46 M).
-size_t renderNoiseEntries() {
+const size_t kRenderNoiseEntries = [] {
     size_t total = 0;
     for (int k = 0; k < kRenderTables; ++k) {
         const int f = k / kRenderOctaves, o = k % kRenderOctaves;
         total += static_cast<size_t>(renderTableSize(f, o, 0)) * renderTableSize(f, o, 1) * renderTableSize(f, o, 2);
     }
     return total;
-}
+}();
 
 }  // namespace
 
@@ -1111,7 +1111,7 @@ size_t renderNoiseEntries() {
 // kLatticeReach has none.  They lie in the force scratch, which no stage of a
 // frame uses, where the grid has the cells for them, else in renderNoise_.
 bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
-    float4* room = cells_ >= renderNoiseEntries() ? contrib_ : renderNoise_;
+    float4* room = cells_ >= kRenderNoiseEntries ? contrib_ : renderNoise_;
     if (!latticesEnabled_ || room == nullptr) return false;
     const double t = p.time;
     const double lo[4][3] = {{t * 0.18, -t * 0.11, t * 0.07}, {-t * 0.14, t * 0.10, -t * 0.08}, {t * 0.72, -t * 1.28, t * 0.38},
@@ -1142,28 +1142,26 @@ bool Scene::renderNoise(const FrameParams& p, RenderNoise& n) {
     return true;
 }
 
+bool Scene::needsRenderNoise() const {
+    return physics_.mode == 0 && cells_ < kRenderNoiseEntries && renderNoise_ == nullptr && !renderNoiseRefused_;
+}
+
+size_t Scene::deviceBytes() const {
+    return deviceBytes_ + (renderNoiseOnUse_ && needsRenderNoise() ? kRenderNoiseEntries * sizeof(float4) : 0);
+}
+
 void Scene::placeRenderNoise() {
-    const bool wanted = physics_.mode == 0 && cells_ < renderNoiseEntries();
-    if (wanted == (renderNoise_ != nullptr) || (wanted && renderNoiseRefused_)) return;
+    if (!needsRenderNoise()) return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamIsCapturing(stream, &capture) != cudaSuccess ||
-        capture != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return;
     }
-    const size_t bytes = renderNoiseEntries() * sizeof(float4);
-    if (wanted) {
-        std::string ignored;
-        if (!alloc(reinterpret_cast<void**>(&renderNoise_), bytes, "cudaMalloc render noise", ignored)) {
-            cudaGetLastError();
-            renderNoiseRefused_ = true;
-        }
-        return;
+    std::string ignored;
+    if (!alloc(reinterpret_cast<void**>(&renderNoise_), kRenderNoiseEntries * sizeof(float4), "cudaMalloc render noise", ignored)) {
+        cudaGetLastError();
+        renderNoiseRefused_ = true;
     }
-    cudaStreamSynchronize(stream);  // frames that read them may be queued
-    deviceFree(renderNoise_);
-    renderNoise_ = nullptr;
-    deviceBytes_ -= bytes;
 }
 
 bool Scene::runStages(int first, int last, const FrameParams& p, std::string& err) {
@@ -1172,6 +1170,7 @@ bool Scene::runStages(int first, int last, const FrameParams& p, std::string& er
         return false;
     }
     if (physics_.mode == 1) return runConfigStages(first, last, p, err);
+    if (renderNoiseOnUse_ && first <= kRender) placeRenderNoise();
     const int bx = rowThreads(nx);
     const dim3 cells = cellGrid(bx, nx, ny, nz);
     int s = first;

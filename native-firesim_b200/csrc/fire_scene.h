@@ -141,17 +141,19 @@ public:
     // Physics of the following passes (mode 0 reference, mode 1 config physics).
     bool setPhysics(const FirePhysicsParams& params, std::string& err);
     const FirePhysicsParams& physics() const { return physics_; }
-    // Gives a scene of the reference physics the room for its noise tables, and
-    // takes it from one of the config physics, which has none.  Whoever makes the
-    // scene or sets its physics calls this, so that no frame allocates and
-    // deviceBytes() has it beforehand; a scene without the room hashes in place.
+    // Allocates the room of the raymarch's noise tables, if this scene needs one of
+    // its own (needsRenderNoise).  A scene's first step of the reference physics
+    // calls this, so that no frame allocates, unless renderNoiseOnUse(false): then
+    // only whoever made the scene does, or frames hash in place.
     void placeRenderNoise();
+    void renderNoiseOnUse(bool enabled) { renderNoiseOnUse_ = enabled; }
     // Steps of the config physics since the last reset (the emitter jitter's counter).
     unsigned long long configStep() const { return cfgStep_; }
     bool synchronize(std::string& err);
     // After a host sync: fails once with "timed out" if a resident SOR wait ran out since the last check.
     bool checkSolverStatus(std::string& err);
-    size_t deviceBytes() const { return deviceBytes_; }
+    // With the noise tables that the first step will allocate.
+    size_t deviceBytes() const;
     unsigned long long launchCount() const { return launches_; }
 
     int nx = 0, ny = 0, nz = 0, lnx = 0, lny = 0, lnz = 0, frameW = 0, frameH = 0, device = 0;
@@ -227,9 +229,11 @@ private:
     float* sourceLattice_ = nullptr;
     size_t sourceCapacity_ = 0;
     // Hash tables of the raymarch's noise fields, where the force scratch has no room
-    // for them (placeRenderNoise); null: frames hash in place.
+    // for them; null: frames hash in place.
     bool renderNoise(const FrameParams& p, RenderNoise& n);
+    bool needsRenderNoise() const;
     float4* renderNoise_ = nullptr;
+    bool renderNoiseOnUse_ = true;
     bool renderNoiseRefused_ = false;  // their allocation failed
     // Raymarch work list: tile order (centre first) and the tile counter.
     int* rayTileOrder_ = nullptr;

@@ -68,7 +68,6 @@ extern "C" FireScene* fireSceneCreate(int device, int frameW, int frameH, int nx
         fail(err);
         return nullptr;
     }
-    scene->placeRenderNoise();
     FireScene* h = new FireScene;
     h->scene = std::move(scene);
     h->device = device;
@@ -102,7 +101,6 @@ extern "C" bool fireSceneSetPhysicsParams(FireScene* scene, const FirePhysicsPar
     if (params == nullptr) return fail("Physics parameter pointer was null.");
     std::string err;
     if (!scene->scene->setPhysics(*params, err)) return fail(err);
-    scene->scene->placeRenderNoise();
     return true;
 }
 
@@ -669,8 +667,9 @@ extern "C" bool fireServerRun(FireServer* server, double maxSeconds, FireServeRe
                     break;
                 }
                 // The noise tables of a scene that renders the reference physics, before it is
-                // counted: no frame allocates.  (A pooled scene that was made for another
+                // counted: no step allocates.  (A pooled scene that was made for another
                 // request may be without them and hashes in place.)
+                a->scene->renderNoiseOnUse(false);
                 if (r.physics.mode == 0 && r.renderEvery > 0) a->scene->placeRenderNoise();
                 a->bytes = a->scene->deviceBytes() + frameBytes(r);
                 server->bytesByShape[shape] = a->bytes;

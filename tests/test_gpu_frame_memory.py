@@ -1,6 +1,7 @@
-"""The raymarch's noise tables are part of a scene from its making on (needs a
-GPU): no frame changes what a scene holds, a served scene is counted with them
-before it is admitted, and the config physics, which has none, gives them back."""
+"""The raymarch's noise tables count as a scene's memory from its making on (needs a
+GPU): neither a step nor a frame changes what a scene reports, a served scene is
+counted with them before it is admitted, and a scene of the config physics, which
+has none, never allocates them."""
 from __future__ import annotations
 
 import pytest
@@ -26,18 +27,29 @@ def test_no_frame_changes_what_a_scene_holds(pkg, abi):
     hdr = torch.zeros((48, 64, 4), device="cuda")
     scene = pkg.Scene(64, 48, *DIMS)
     made = scene.device_bytes()
-    _frame(pkg, abi, scene, hdr, 1)
+    s = abi.validation_settings(0, width=64, height=48)
+    scene.step(s, render=False)
     assert scene.device_bytes() == made
+    free = torch.cuda.mem_get_info()[0]
+    _frame(pkg, abi, scene, hdr, 0)
+    # (A kernel's first launch loads its code, a few MB; the tables are 23 MB.)
+    assert free - torch.cuda.mem_get_info()[0] < 20_000_000
+    assert scene.device_bytes() == made
+    scene.close()
+
+
+def test_the_config_physics_has_no_tables(pkg, abi):
+    scene = pkg.Scene(64, 48, *DIMS)
+    made = scene.device_bytes()
     p = abi.default_physics(*DIMS)
     p.mode = 1
     scene.set_physics(p)
-    without = scene.device_bytes()
-    assert made - without > 20_000_000
+    assert made - scene.device_bytes() > 20_000_000
+    scene.step(abi.FireSettings(width=64, height=48, reset=1), render=False)
+    assert scene.device_bytes() < made
     p.mode = 0
     scene.set_physics(p)
-    assert scene.device_bytes() == made
-    _frame(pkg, abi, scene, hdr, 1)
-    assert scene.device_bytes() == made
+    assert scene.device_bytes() > made
     scene.close()
 
 
