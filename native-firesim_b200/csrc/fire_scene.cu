@@ -1157,11 +1157,16 @@ void Scene::placeRenderNoise() {
         cudaGetLastError();
         return;
     }
+    // Some other stream may be in a capture that an allocation would end, unless this
+    // thread says that it does not concern it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     std::string ignored;
     if (!alloc(reinterpret_cast<void**>(&renderNoise_), kRenderNoiseEntries * sizeof(float4), "cudaMalloc render noise", ignored)) {
         cudaGetLastError();
         renderNoiseRefused_ = true;
     }
+    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 bool Scene::runStages(int first, int last, const FrameParams& p, std::string& err) {

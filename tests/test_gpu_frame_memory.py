@@ -53,6 +53,31 @@ def test_the_config_physics_has_no_tables(pkg, abi):
     scene.close()
 
 
+def test_the_tables_do_not_end_a_capture_elsewhere(pkg, abi):
+    import numpy as np
+    import torch
+
+    frames = []
+    x = torch.zeros(8, device="cuda")
+    for capture in (False, True):
+        sim = pkg.FireSim(64, 48, *DIMS)
+        s = abi.validation_settings(3, width=64, height=48)
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, capture_error_mode="global"):
+                x += 1.0
+                sim.stages("light_build", "render", s, 0.5, wait=False)
+            graph.replay()
+            torch.cuda.synchronize()
+        else:
+            sim.stages("light_build", "render", s, 0.5)
+        sim.synchronize()
+        frames.append(sim.get("hdr"))
+        sim.close()
+    assert float(x[0]) == 1.0
+    assert np.array_equal(frames[0].view(np.uint32), frames[1].view(np.uint32))
+
+
 def test_server_counts_a_scene_as_it_is_after_a_frame(pkg, abi):
     import torch
 
