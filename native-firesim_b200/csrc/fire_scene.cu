@@ -2004,6 +2004,7 @@ namespace {
 constexpr long long kLightLaneRays = 32768;
 bool pixelLanes(const ConfigParams& c, size_t cells, bool skips) {
     const long long rays = static_cast<long long>(c.frameW) * c.frameH;
+    if (c.frameH > 2 * 65535) return false;  // its grid has a row of blocks for two rows of pixels
     return rays <= 36864 || (rays <= std::min(131072LL, 1024LL * c.primarySamples) && (skips || cells <= 4000000));
 }
 }  // namespace

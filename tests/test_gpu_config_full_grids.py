@@ -57,3 +57,17 @@ def test_full_and_empty_grids_with_many_samples(pkg, abi, dims, samples, kind):
     sim.close()
     for x, y in zip(a, b):
         assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
+
+
+def test_a_frame_of_one_column(pkg, abi):
+    """131,072 rays in one column: more rows than a grid of two-row blocks has."""
+    sim = pkg.FireSim(1, 131072, 24, 20, 16)
+    p = abi.default_physics(24, 20, 16)
+    p.mode, p.primarySamples = 1, 128
+    sim.set_physics(p)
+    sim.reset()
+    sim.set("soot", np.full((16, 20, 24), 0.5, np.float32))
+    sim.stages("light_build", "render", abi.FireSettings(width=1, height=131072), 0.0)
+    hdr = sim.get("hdr")
+    sim.close()
+    assert np.isfinite(hdr).all() and hdr[..., 3].max() > 0.5
